@@ -403,9 +403,9 @@ magma_int_t magma_b200_host_solver_destroy(magma_b200_host_solver_t solver);
  * .f64 (bit-identical to 0-2) and FP32 128x128 with tcgen05 split TF32 (within the
  * reference tester's 30 eps bound, not bit-identical to 0-2)) for
  * max(M,N) <= 16, <= 32, <= 64 and larger, first for FP64 then FP32; 1/0 for the
- * tensor-core LU in magma_dsgesv_batched (n = 96..256, step 32) as a whole; 1/0 for
- * the FP64 blocked LU's trailing update on the tensor cores (DMMA) instead of the
- * FP64 pipe, for max(m) <= 128, <= 256, <= 512, <= 1024; and 1/0 for the tensor-core
+ * tensor-core LU in magma_dsgesv_batched (n = 96..256, step 32) as a whole; four 0/1
+ * values that are no longer read (once the FP64 blocked LU's update variant for max(m)
+ * <= 128, <= 256, <= 512, <= 1024); and 1/0 for the tensor-core
  * LU (with its fused refinement) at each order n = 96, 128, ..., 256; 1/0 for the
  * variable-size FP64 Cholesky (potrf / potrs / posv vbatched) as one persistent
  * launch over all orders <= 512 instead of one launch per size bucket; and 1/0 for

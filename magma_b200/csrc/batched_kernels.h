@@ -21,10 +21,14 @@ template <typename T>
 magma_int_t getrs_small(const WorkList& wl, int bound, bool persistent, bool trans, const LuSizes& sz, int max_n,
                         int max_nrhs, T** A, int** ipiv, T** B, cudaStream_t s);
 
-// Blocked LU family (getrf_blocked.cu): one matrix per thread block, m <= 1024.
+// Blocked LU family (getrf_blocked.cu), m <= 1024: one matrix per thread block, or in FP64
+// getrf per thread-block cluster.
 bool blocked_lu_supported(int max_m);
 template <typename T>
 magma_int_t getrf_blocked(const WorkList& wl, int bound, bool persistent, const LuSizes& sz, int max_m, T** A,
+                          int** ipiv, int* info, cudaStream_t s);
+// FP64 LU, one matrix per thread-block cluster (getrf_cluster.cu): m <= 1024.
+magma_int_t getrf_cluster(const WorkList& wl, int bound, bool persistent, const LuSizes& sz, int max_m, double** A,
                           int** ipiv, int* info, cudaStream_t s);
 template <typename T>
 magma_int_t getrs_blocked(const WorkList& wl, int bound, bool persistent, bool trans, const LuSizes& sz, int max_n,

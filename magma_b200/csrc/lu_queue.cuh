@@ -49,7 +49,7 @@ template <typename T, int R>
 struct LuQueueShare {
     template <int S>
     static constexpr size_t per_warp() {
-        constexpr size_t f = sizeof(BlockedLuShared<T, 32, S, LuQueueTeam<S>::CW, false>);
+        constexpr size_t f = sizeof(BlockedLuShared<T, 32, S, LuQueueTeam<S>::CW>);
         constexpr size_t s = sizeof(BlockedRsShared<T, S, R>);
         return ((f > s ? f : s) + S / 32 - 1) / (S / 32);
     }
@@ -70,9 +70,9 @@ __device__ __forceinline__ void lu_queue_blocked(int id, const LuSizes& sz, T** 
     using TT = LuQueueTeam<S>;
     const int m = sz.get_m(id), n = sz.get_n(id), lda = sz.get_lda(id);
     int* ipiv = ipiv_array ? ipiv_array[id] : nullptr;   // null: LU without pivoting
-    auto& sh = *reinterpret_cast<BlockedLuShared<T, 32, S, TT::CW, false>*>(base);
+    auto& sh = *reinterpret_cast<BlockedLuShared<T, 32, S, TT::CW>*>(base);
     int info = 0;
-    blocked_getrf<T, 32, S, TT::CW, TT::CB, false>(dA[id], m, n, lda, ipiv, info, sh, team);
+    blocked_getrf<T, 32, S, TT::CW, TT::CB>(dA[id], m, n, lda, ipiv, info, sh, team);
     if (team.tid() == 0) info_array[id] = info;
     team.sync();   // the solve's shared memory overlays the factorisation's
     if constexpr (SOLVE) {

@@ -37,9 +37,7 @@ static void set_defaults(TuningTable& t) {
         for (int b = 0; b < kGemmBuckets; ++b) t.gemm_variant[p][b] = gemm[p][b];
     const char* e = std::getenv("MAGMA_B200_TENSOR_CORE_LU");
     t.mixed_tc_lu = (e && e[0] == '0') ? 0 : 1;
-    // the FP64 pipe's update in every bucket (DMMA is slower at each size: n = 256
-    // 684 against 734 us in ncu, 1,024 within noise)
-    for (int b = 0; b < kLuBlockedBuckets; ++b) t.lu_dmma[b] = 0;
+    for (int b = 0; b < kUnusedValues; ++b) t.unused[b] = 0;
     // tensor-core LU from n = 160 on; the CUDA-core FP32 LU is faster at n = 96 and 128
     for (int i = 0; i < kMixedTcOrders; ++i) t.mixed_tc_n[i] = (i >= 2);
     t.chol_queue = 1;   // one launch for the variable-size Cholesky
@@ -51,7 +49,7 @@ static void to_values(const TuningTable& t, int* v) {
     for (int p = 0; p < 2; ++p)
         for (int b = 0; b < kGemmBuckets; ++b) v[i++] = t.gemm_variant[p][b];
     v[i++] = t.mixed_tc_lu;
-    for (int b = 0; b < kLuBlockedBuckets; ++b) v[i++] = t.lu_dmma[b];
+    for (int b = 0; b < kUnusedValues; ++b) v[i++] = t.unused[b];
     for (int k = 0; k < kMixedTcOrders; ++k) v[i++] = t.mixed_tc_n[k];
     v[i++] = t.chol_queue;
     v[i++] = t.lu_queue;
@@ -72,7 +70,7 @@ static bool from_values(const int* v, int count, TuningTable& t) {
         for (int b = 0; b < kGemmBuckets; ++b) t.gemm_variant[p][b] = v[i++];
     t.mixed_tc_lu = v[i++];
     if (count >= kTuningValuesV2)
-        for (int b = 0; b < kLuBlockedBuckets; ++b) t.lu_dmma[b] = v[i++];
+        for (int b = 0; b < kUnusedValues; ++b) t.unused[b] = v[i++];
     if (count >= kTuningValuesV3)
         for (int k = 0; k < kMixedTcOrders; ++k) t.mixed_tc_n[k] = v[i++];
     if (count >= kTuningValuesV4) t.chol_queue = v[i++];
@@ -279,45 +277,6 @@ static magma_int_t tune_mixed(magma_queue_t q, unsigned seed) {
     return MAGMA_SUCCESS;
 }
 
-// FP64 blocked LU: for each bucket, the two trailing-update variants on a batch of
-// about 256 MB of uniform[-1,1] matrices of the bucket's largest order, through
-// magma_dgetrf_batched (both variants give bit-identical factors).
-static magma_int_t tune_lu_update(magma_queue_t q, unsigned seed) {
-    const int orders[kLuBlockedBuckets] = {128, 256, 512, 1024};
-    for (int b = 0; b < kLuBlockedBuckets; ++b) {
-        const int n = orders[b];
-        const int batch = std::max(16, (256 << 20) / (8 * n * n));
-        const size_t an = (size_t)n * n * batch;
-        DevBuf dA, dA0, dP, dI;
-        if (!dA.alloc(8 * an) || !dA0.alloc(8 * an) || !dP.alloc(sizeof(void*) * 2 * batch) ||
-            !dI.alloc(sizeof(int) * ((size_t)n * batch + batch)))
-            return MAGMA_ERR_DEVICE_ALLOC;
-        tune_fill_kernel<double><<<1024, 256, 0, q->stream>>>((double*)dA0.p, an, seed + b);
-        std::vector<void*> ptr(2 * batch);
-        for (int i = 0; i < batch; ++i) {
-            ptr[i] = (double*)dA.p + (size_t)i * n * n;
-            ptr[batch + i] = (int*)dI.p + (size_t)i * n;
-        }
-        cudaMemcpyAsync(dP.p, ptr.data(), sizeof(void*) * 2 * batch, cudaMemcpyHostToDevice, q->stream);
-        cudaStreamSynchronize(q->stream);
-        void** p = (void**)dP.p;
-        int* info = (int*)dI.p + (size_t)n * batch;
-        float best = 1e30f;
-        int best_v = tuning().lu_dmma[b];
-        for (int v = 0; v < 2; ++v) {
-            tuning_mut().lu_dmma[b] = v;
-            const float ms = time_ms(q->stream, [&] {
-                cudaMemcpyAsync(dA.p, dA0.p, 8 * an, cudaMemcpyDeviceToDevice, q->stream);
-                magma_dgetrf_batched(n, n, (double**)p, n, (int**)(p + batch), info, batch, q);
-            }, 3);
-            if (cudaGetLastError() != cudaSuccess) return MAGMA_ERR_UNKNOWN;
-            if (ms < best) { best = ms; best_v = v; }
-        }
-        tuning_mut().lu_dmma[b] = best_v;
-    }
-    return MAGMA_SUCCESS;
-}
-
 // Sets each n x n matrix's diagonal to 2n + its value: with the other lower-triangle
 // entries in [-1, 1) the symmetric matrix the lower triangle defines is diagonally
 // dominant, hence positive definite.
@@ -470,7 +429,6 @@ magma_int_t magma_b200_autotune(magma_queue_t queue) {
     magma_int_t rc = tune_gemm<double>(0, queue, 17);
     if (!rc) rc = tune_gemm<float>(1, queue, 23);
     if (!rc) rc = tune_mixed(queue, 29);
-    if (!rc) rc = tune_lu_update(queue, 31);
     if (!rc) rc = tune_chol_queue(queue, 37);
     if (!rc) rc = tune_lu_queue(queue, 41);
     cudaStreamSynchronize(queue->stream);
