@@ -30,6 +30,9 @@ magma_int_t getrf_blocked(const WorkList& wl, int bound, bool persistent, const 
 // FP64 LU, one matrix per thread-block cluster (getrf_cluster.cu): m <= 1024.
 magma_int_t getrf_cluster(const WorkList& wl, int bound, bool persistent, const LuSizes& sz, int max_m, double** A,
                           int** ipiv, int* info, cudaStream_t s);
+// FP64 solves of those orders on the tensor cores (getrs_tc.cu).
+magma_int_t getrs_tc(const WorkList& wl, int bound, bool persistent, bool trans, const LuSizes& sz, int max_n,
+                     int max_nrhs, double** A, int** ipiv, double** B, cudaStream_t s);
 template <typename T>
 magma_int_t getrs_blocked(const WorkList& wl, int bound, bool persistent, bool trans, const LuSizes& sz, int max_n,
                           int max_nrhs, T** A, int** ipiv, T** B, cudaStream_t s);

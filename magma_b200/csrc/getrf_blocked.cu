@@ -1,6 +1,6 @@
 // getrf_blocked.cu -- kernels and host dispatch of the blocked batched LU
-// (one matrix per thread block, up to 1024 rows): FP32 getrf, and getrs. FP64 getrf of
-// these orders is getrf_cluster.cu.
+// (one matrix per thread block, up to 1024 rows): FP32. FP64 runs getrf_cluster.cu
+// and getrs_tc.cu.
 #include "internal.h"
 #include "blocked_lu.cuh"
 #include "getrs_blocked.cuh"
@@ -94,11 +94,15 @@ static void launch_getrs_blocked(const WorkList& wl, int bound, bool persistent,
 template <typename T>
 magma_int_t getrs_blocked(const WorkList& wl, int bound, bool persistent, bool trans, const LuSizes& sz, int max_n,
                           int max_nrhs, T** A, int** ipiv, T** B, cudaStream_t s) {
-    if (max_n <= 128) launch_getrs_blocked<T, 128>(wl, bound, persistent, sz, trans, max_nrhs, A, ipiv, B, s);
-    else if (max_n <= 256) launch_getrs_blocked<T, 256>(wl, bound, persistent, sz, trans, max_nrhs, A, ipiv, B, s);
-    else if (max_n <= 512) launch_getrs_blocked<T, 512>(wl, bound, persistent, sz, trans, max_nrhs, A, ipiv, B, s);
-    else launch_getrs_blocked<T, 1024>(wl, bound, persistent, sz, trans, max_nrhs, A, ipiv, B, s);
-    return launch_status();
+    if constexpr (std::is_same<T, double>::value) {
+        return getrs_tc(wl, bound, persistent, trans, sz, max_n, max_nrhs, A, ipiv, B, s);
+    } else {
+        if (max_n <= 128) launch_getrs_blocked<T, 128>(wl, bound, persistent, sz, trans, max_nrhs, A, ipiv, B, s);
+        else if (max_n <= 256) launch_getrs_blocked<T, 256>(wl, bound, persistent, sz, trans, max_nrhs, A, ipiv, B, s);
+        else if (max_n <= 512) launch_getrs_blocked<T, 512>(wl, bound, persistent, sz, trans, max_nrhs, A, ipiv, B, s);
+        else launch_getrs_blocked<T, 1024>(wl, bound, persistent, sz, trans, max_nrhs, A, ipiv, B, s);
+        return launch_status();
+    }
 }
 
 template magma_int_t getrf_blocked<double>(const WorkList&, int, bool, const LuSizes&, int, double**, int**, int*,
