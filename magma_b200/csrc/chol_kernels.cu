@@ -2,6 +2,7 @@
 // their host launchers. Device code in chol.cuh.
 #include "internal.h"
 #include "chol.cuh"
+#include "chol_team.cuh"
 #include "lu_sizes.h"
 #include "vbatched.h"
 #include "chol_launch.h"
@@ -69,6 +70,32 @@ potrs_blocked_kernel(WorkList wl, LuSizes sz, bool upper, T** dA_array, T** dB_a
     }
 }
 
+// ---- FP64 potrf (n <= S) / potrs (n <= ROWS) by a block of S threads ----
+template <int S>
+__global__ void __launch_bounds__(S, (S <= 128 ? 4 : S == 256 ? 2 : 1))
+potrf_team_kernel(WorkList wl, LuSizes sz, bool upper, double** dA_array, int* info_array) {
+    const BlockTeam team;
+    for (int w = blockIdx.x; w < wl.size(); w += gridDim.x) {
+        const int id = wl.at(w), n = sz.get_n(id);
+        int info = 0;
+        if (n > 0) info = chol_team_potrf(dA_array[id], n, sz.get_lda(id), upper, 0u, S, team);
+        if (threadIdx.x == 0 && info_array) info_array[id] = info;
+        __syncthreads();
+    }
+}
+
+template <int S, int ROWS>
+__global__ void __launch_bounds__(S, (S == 64 ? 5 : S == 128 ? 4 : 2))
+potrs_team_kernel(WorkList wl, LuSizes sz, bool upper, double** dA_array, double** dB_array) {
+    const BlockTeam team;
+    for (int w = blockIdx.x; w < wl.size(); w += gridDim.x) {
+        const int id = wl.at(w), n = sz.get_n(id);
+        if (n > 0)
+            chol_team_potrs(dA_array[id], n, sz.get_lda(id), upper, dB_array[id], sz.get_nrhs(id), sz.get_ldb(id),
+                            0u, S, ROWS, blockIdx.y, gridDim.y, team);
+    }
+}
+
 // ---------------------------------------------------------------------------
 // Launchers. Each bucket launcher covers instances with n in (lo, hi].
 template <typename K>
@@ -120,6 +147,13 @@ static void launch_potrs_small(const WorkList& wl, int bound, bool persistent, c
 template <typename T, int NB, int NT, int CW, int CB>
 static void launch_potrf_blocked(const WorkList& wl, int bound, bool persistent, const LuSizes& sz, bool upper,
                                  T** A, int* info, cudaStream_t s) {
+    if constexpr (std::is_same<T, double>::value && NT <= 512) {
+        auto k = potrf_team_kernel<NT>;
+        const int smem = (int)chol_team_smem(NT);
+        ensure_dynamic_smem((const void*)k, smem);
+        k<<<grid_for(k, NT, bound, persistent, smem), NT, smem, s>>>(wl, sz, upper, A, info);
+        return;
+    }
     auto k = potrf_blocked_kernel<T, NB, NT, CW, CB>;
     const int smem = (int)sizeof(BlockedCholShared<T, NB, NT, CW>);
     ensure_dynamic_smem((const void*)k, smem);
@@ -129,6 +163,15 @@ static void launch_potrf_blocked(const WorkList& wl, int bound, bool persistent,
 template <typename T, int NT>
 static void launch_potrs_blocked(const WorkList& wl, int bound, bool persistent, const LuSizes& sz, bool upper,
                                  T** A, T** B, int max_nrhs, cudaStream_t s) {
+    if constexpr (std::is_same<T, double>::value) {
+        constexpr int S = NT < 256 ? NT / 2 : NT == 256 ? 128 : 256;   // as the LU solves (getrs_tc.cu)
+        auto k = potrs_team_kernel<S, NT>;
+        const int smem = (int)(sizeof(double) * kTriRhs * NT + sizeof(TriStage));
+        ensure_dynamic_smem((const void*)k, smem);
+        const int gy = min(4, ceildiv(max(1, max_nrhs), kTriRhs));
+        k<<<dim3(grid_for(k, S, bound, persistent, smem), gy), S, smem, s>>>(wl, sz, upper, A, B);
+        return;
+    }
     if (max_nrhs <= 1) {
         auto k = potrs_blocked_kernel<T, NT, 1>;
         k<<<grid_for(k, NT, bound, persistent), NT, 0, s>>>(wl, sz, upper, A, B);

@@ -10,7 +10,7 @@ template <typename T, bool FACTOR, bool SOLVE, int R>
 static void launch_queue(const CholQueue& q, int bound, const LuSizes& sz, bool upper, T** A, T** B, int* info,
                          cudaStream_t s) {
     auto k = chol_queue_kernel<T, FACTOR, SOLVE, R>;
-    const size_t smem = QueueShare<T, R>::bytes * kQueueWarps;
+    const size_t smem = QueueShare<T>::bytes * kQueueWarps;
     ensure_dynamic_smem((const void*)k, (int)smem);
     const int grid = max(1, min(bound, resident_blocks((const void*)k, kQueueThreads, smem)));
     k<<<grid, kQueueThreads, smem, s>>>(q, sz, upper, A, B, info);

@@ -8,7 +8,7 @@
 // warps. A team that draws an instance needing fewer threads splits in two: the
 // lower half keeps the instance, the upper half draws the next ticket. Teams
 // therefore only ever split, down to single warps:
-//   512 threads  256 < n <= 512   blocked potrf (thread = row) + blocked potrs
+//   512 threads  256 < n <= 512   blocked potrf + potrs of a team (chol_team.cuh)
 //   256          128 < n <= 256
 //   128           64 < n <= 128
 //    64           32 < n <=  64
@@ -19,14 +19,15 @@
 // for a loop of their own (tickets by shuffle): keeping the two loops apart keeps
 // the register-resident small path from spilling under the block's 128 registers.
 //
-// Each instance runs the same device functions, in the same thread-per-row
-// layout, as the per-bucket kernels of chol_kernels.cu, so the results are the
-// same bits. Counterparts in the reference: src/zpotrf_vbatched.cpp:146-204 (a
+// Each instance runs the same device functions as the per-bucket kernels of
+// chol_kernels.cu (orders 33..64 the team code instead of the two-warp register kernel),
+// so the results are the same bits. Counterparts in the reference: src/zpotrf_vbatched.cpp:146-204 (a
 // launch sequence per size class) and magmablas/gemm_template_kernel_vbatched.cuh:53-54
 // (grids sized by the largest instance, smaller instances' blocks exit early).
 #pragma once
 
 #include "chol.cuh"
+#include "chol_team.cuh"
 #include "chol_launch.h"
 #include "lu_sizes.h"
 
@@ -46,19 +47,13 @@ struct CholQueue {
     int* head;
 };
 
-template <size_t A, size_t B> struct MaxSz { static constexpr size_t v = A > B ? A : B; };
-
 // Shared memory of one warp's share: the largest per-warp need over the team sizes.
-template <typename T, int R>
+template <typename T>
 struct QueueShare {
-    template <int S>
-    static constexpr size_t per_warp() {
-        constexpr size_t f = sizeof(BlockedCholShared<T, 32, S, 64>), s = sizeof(BlockedCholRsShared<T, S, R>);
-        return ((f > s ? f : s) + S / 32 - 1) / (S / 32);
-    }
-    static constexpr size_t raw =
-        MaxSz<MaxSz<sizeof(CholShared<T, 32>), per_warp<64>()>::v,
-              MaxSz<per_warp<128>(), MaxSz<per_warp<256>(), per_warp<512>()>::v>::v>::v;
+    static constexpr size_t per_warp(int S) { return (chol_team_smem(S) + S / 32 - 1) / (S / 32); }
+    static constexpr size_t max2(size_t a, size_t b) { return a > b ? a : b; }
+    static constexpr size_t raw = max2(max2(sizeof(CholShared<T, 32>), per_warp(64)),
+                                       max2(per_warp(128), max2(per_warp(256), per_warp(512))));
     static constexpr size_t bytes = (raw + 15) / 16 * 16;
 };
 
@@ -71,28 +66,20 @@ __device__ __forceinline__ void queue_team_sync(int S, int w0) {
     else BarSync{queue_team_barrier_id(S, w0), S}();
 }
 
-// One instance on a team of S threads (S >= 64): blocked potrf, then potrs.
-template <typename T, int S, bool FACTOR, bool SOLVE, int R>
-__device__ __forceinline__ void queue_blocked(int id, const LuSizes& sz, bool upper, T** dA, T** dB, int* info,
-                                              unsigned char* base, const WarpRangeTeam& team) {
+// One instance on a team of S threads (S >= 64): blocked potrf, then potrs. One code for every
+// team size.
+template <bool FACTOR, bool SOLVE>
+__device__ __forceinline__ void queue_blocked(int id, const LuSizes& sz, bool upper, double** dA, double** dB,
+                                              int* info, unsigned off, int S, const WarpRangeTeam& team) {
     const int n = sz.get_n(id), lda = sz.get_lda(id);
     if constexpr (FACTOR) {
-        auto& sh = *reinterpret_cast<BlockedCholShared<T, 32, S, 64>*>(base);
-        // FP64 teams of 256 and 512 threads: the trailing updates on the tensor cores (the same
-        // bits as the CUDA-core form, which the smaller teams keep: with them as well the
-        // kernel spills heavily under its 128 registers)
-        constexpr bool kDmma = std::is_same<T, double>::value && S >= 256;
-        const int inf = blocked_potrf<T, 32, S, 64, 8, WarpRangeTeam, kDmma, false>(dA[id], n, lda, upper, sh, team);
+        const int inf = chol_team_potrf(dA[id], n, lda, upper, off, S, team);
         if (team.tid() == 0 && info) info[id] = inf;
         team.sync();   // the solve's shared memory overlays the factor's
     }
     if constexpr (SOLVE) {
         // MAGMA's posv solves regardless of info (src/zposv_batched.cpp:123-141)
-        const int nrhs = sz.get_nrhs(id);
-        if (nrhs > 0) {
-            auto& rs = *reinterpret_cast<BlockedCholRsShared<T, S, R>*>(base);
-            blocked_potrs<T, S, R>(dA[id], n, lda, upper, dB[id], nrhs, sz.get_ldb(id), rs, team);
-        }
+        chol_team_potrs(dA[id], n, lda, upper, dB[id], sz.get_nrhs(id), sz.get_ldb(id), off, S, S, 0, 1, team);
     }
 }
 
@@ -120,7 +107,7 @@ chol_queue_kernel(CholQueue q, LuSizes sz, bool upper, T** dA, T** dB, int* info
     extern __shared__ __align__(16) unsigned char queue_smem[];
     __shared__ int drawn[kQueueWarps];
     __shared__ int first[kQueueBuckets], count[kQueueBuckets];
-    constexpr size_t share = QueueShare<T, R>::bytes;
+    constexpr size_t share = QueueShare<T>::bytes;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
         int t = 0;
@@ -158,14 +145,9 @@ chol_queue_kernel(CholQueue q, LuSizes sz, bool upper, T** dA, T** dB, int* info
             }
             continue;
         }
-        unsigned char* base = queue_smem + (size_t)w0 * share;
+        const unsigned off = (unsigned)(w0 * share);
         const WarpRangeTeam team{w0 * 32, queue_team_barrier_id(S, w0), S};
-        switch (S) {
-            case 512: queue_blocked<T, 512, FACTOR, SOLVE, R>(id, sz, upper, dA, dB, info, base, team); break;
-            case 256: queue_blocked<T, 256, FACTOR, SOLVE, R>(id, sz, upper, dA, dB, info, base, team); break;
-            case 128: queue_blocked<T, 128, FACTOR, SOLVE, R>(id, sz, upper, dA, dB, info, base, team); break;
-            default: queue_blocked<T, 64, FACTOR, SOLVE, R>(id, sz, upper, dA, dB, info, base, team); break;
-        }
+        queue_blocked<FACTOR, SOLVE>(id, sz, upper, dA, dB, info, off, S, team);
         t = -1;
     }
     // single warps (n <= 32): registers; the ticket travels by shuffle

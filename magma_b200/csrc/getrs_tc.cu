@@ -13,7 +13,7 @@ namespace mb200 {
 // Dynamic shared memory: X (NMAX x 8), the two staged blocks, the pivots.
 template <int NMAX>
 constexpr size_t getrs_tc_smem() {
-    return sizeof(double) * NMAX * kTriRhs + 2 * sizeof(TriDiagShared) + sizeof(int) * NMAX;
+    return sizeof(double) * NMAX * kTriRhs + sizeof(TriStage) + sizeof(int) * NMAX;
 }
 
 template <int NMAX, int NT>
@@ -22,8 +22,8 @@ getrs_tc_kernel(WorkList wl, LuSizes sz, bool trans, double** dA_array, int** ip
     constexpr int NW = NT / 32, RPT = NMAX / NT;
     extern __shared__ __align__(16) unsigned char getrs_tc_raw[];
     double* X = reinterpret_cast<double*>(getrs_tc_raw);
-    auto& dg = *reinterpret_cast<TriDiagShared(*)[2]>(X + NMAX * kTriRhs);
-    int* piv = reinterpret_cast<int*>(dg + 2);
+    TriStage& dg = *reinterpret_cast<TriStage*>(X + NMAX * kTriRhs);
+    int* piv = reinterpret_cast<int*>(&dg + 1);
     const BlockTeam team;
     const int tid = threadIdx.x;
     for (int w = blockIdx.x; w < wl.size(); w += gridDim.x) {
@@ -61,11 +61,11 @@ getrs_tc_kernel(WorkList wl, LuSizes sz, bool trans, double** dA_array, int** ip
             }
             __syncthreads();
             if (!trans) {
-                tri_sweep<TriDiag::Unit, false, NW>(A, 1, lda, n, X, dg, team);
-                tri_sweep<TriDiag::Divide, true, NW>(A, 1, lda, n, X, dg, team);
+                tri_sweep<TriDiag::Unit, false>(A, 1, lda, n, X, dg, NW, team);
+                tri_sweep<TriDiag::Divide, true>(A, 1, lda, n, X, dg, NW, team);
             } else {   // U^T (lower), then L^T (upper)
-                tri_sweep<TriDiag::Divide, false, NW>(A, lda, 1, n, X, dg, team);
-                tri_sweep<TriDiag::Unit, true, NW>(A, lda, 1, n, X, dg, team);
+                tri_sweep<TriDiag::Divide, false>(A, lda, 1, n, X, dg, NW, team);
+                tri_sweep<TriDiag::Unit, true>(A, lda, 1, n, X, dg, NW, team);
             }
 #pragma unroll
             for (int j = 0; j < RPT; ++j) {

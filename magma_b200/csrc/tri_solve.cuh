@@ -36,10 +36,15 @@ constexpr int kTriRhs = 8;   // right-hand sides of a sweep
 // Entry (row, col) of X; the swizzle spreads a B fragment's 4 rows x 4 columns over all banks.
 __device__ __forceinline__ int tri_x(int row, int col) { return row * kTriRhs + (col ^ ((row & 2) << 1)); }
 
-struct TriDiagShared {
-    double d[32 * 33];   // the next diagonal block, entry (i, k) at i * 33 + k
-    double p[32 * 33];   // the block of T that couples it to its predecessor
+// The staged blocks of two successive steps: the u-th block in sweep order has its diagonal block
+// in d[u & 1] and the block that couples it to its predecessor in p[(u + 1) & 1], entry (i, k) at
+// tri_e(i, k). A matrix of two blocks never touches p[1].
+struct TriStage {
+    double d[2][1024];
+    double p[2][1024];
 };
+// Swizzled so that A fragments, rows and columns of a block are read and written over all banks.
+__device__ __forceinline__ int tri_e(int i, int k) { return i * 32 + (k ^ (((i & 3) << 2) | ((i >> 2) & 3))); }
 
 // A[0] of the global matrix to shared memory, asynchronously; zero when !valid (nothing is read).
 __device__ __forceinline__ void tri_copy(double* dst, const double* src, bool valid) {
@@ -84,12 +89,12 @@ __device__ __forceinline__ double div_fast(double a, const TriDivisor& v) {
 // The division itself, for the operands div_fast does not take; kept out of the unrolled steps.
 static __device__ __noinline__ double div_slow(double a, double d) { return a / d; }
 
-// One sweep of a team of NW warps (team.sync() is its barrier). T(i, k) = A[i * rs + k * cs];
+// One sweep of a team of NW >= 2 warps (team.sync() is its barrier). T(i, k) = A[i * rs + k * cs];
 // lower and ascending, or upper and descending (DESC). X holds ceil(n / 32) * 32 rows. On entry
 // every warp must see X; on return every warp does.
-template <TriDiag MODE, bool DESC, int NW, typename Team>
-__device__ __forceinline__ void tri_sweep(const double* A, size_t rs, size_t cs, int n, double* X, TriDiagShared (&buf)[2],
-                                          const Team& team) {
+template <TriDiag MODE, bool DESC, typename Team>
+__device__ __forceinline__ void tri_sweep(const double* A, size_t rs, size_t cs, int n, double* X, TriStage& buf,
+                                          int NW, const Team& team) {
     const int tid = team.tid(), lane = tid & 31, warp = tid >> 5;
     const int q = lane & 3, r8 = lane >> 2;
     const int nblk = (n + 31) / 32;
@@ -99,20 +104,20 @@ __device__ __forceinline__ void tri_sweep(const double* A, size_t rs, size_t cs,
 
     // Warps first, first + count, .. : a share of the copies for the u-th block in sweep order.
     auto stage = [&](int u, int share, int shares) {
-        TriDiagShared& dg = buf[u & 1];
+        double *bd = buf.d[u & 1], *bp = buf.p[(u + 1) & 1];
         const int j0 = block_of(u) * 32, p0 = u > 0 ? block_of(u - 1) * 32 : 0;
         for (int e = share; e < 32; e += shares) {
             const int i = rs == 1 ? lane : e, k = rs == 1 ? e : lane;   // lanes along the contiguous direction
             const bool vi = j0 + i < n;
             const bool vd = vi && j0 + k < n, vp = vi && p0 + k < n;
             const double* row = A + (j0 + i) * rs;
-            tri_copy(&dg.d[i * 33 + k], vd ? row + (j0 + k) * cs : A, vd);
-            if (u > 0) tri_copy(&dg.p[i * 33 + k], vp ? row + (p0 + k) * cs : A, vp);
+            tri_copy(&bd[tri_e(i, k)], vd ? row + (j0 + k) * cs : A, vd);
+            if (u > 0) tri_copy(&bp[tri_e(i, k)], vp ? row + (p0 + k) * cs : A, vp);
         }
     };
     // Warp 0: applies the predecessor's solution to the rows of the u-th block and solves them.
     auto lead = [&](int u) {
-        const TriDiagShared& dg = buf[u & 1];
+        const double *bd = buf.d[u & 1], *bp = buf.p[(u + 1) & 1];
         const int j0 = block_of(u) * 32;
         if (u > 0) {
             const int p0 = block_of(u - 1) * 32;
@@ -127,7 +132,7 @@ __device__ __forceinline__ void tri_sweep(const double* A, size_t rs, size_t cs,
             for (int s = 0; s < 8; ++s) {
                 const double b = -X[tri_x(p0 + kof(s), r8)];
 #pragma unroll
-                for (int t = 0; t < 4; ++t) tri_dmma(c[t][0], c[t][1], dg.p[(8 * t + r8) * 33 + kof(s)], b);
+                for (int t = 0; t < 4; ++t) tri_dmma(c[t][0], c[t][1], bp[tri_e(8 * t + r8, kof(s))], b);
             }
 #pragma unroll
             for (int t = 0; t < 4; ++t)
@@ -141,11 +146,11 @@ __device__ __forceinline__ void tri_sweep(const double* A, size_t rs, size_t cs,
             double2 c = *xi;
             double l[8];
 #pragma unroll
-            for (int k = 0; k < 8; ++k) l[k] = dg.d[i * 33 + 8 * t + k];
+            for (int k = 0; k < 8; ++k) l[k] = bd[tri_e(i, 8 * t + k)];
             TriDivisor v;
             bool slow = false;   // a diagonal entry of the piece that div_fast cannot take
             if constexpr (MODE != TriDiag::Unit) {
-                v = tri_divisor(j0 + i < n ? dg.d[i * 33 + i] : 1.0);
+                v = tri_divisor(j0 + i < n ? bd[tri_e(i, i)] : 1.0);
                 if (MODE == TriDiag::Divide) slow = __any_sync(kFullMask, !div_fast_den(v.d));
             }
 #pragma unroll
@@ -182,7 +187,7 @@ __device__ __forceinline__ void tri_sweep(const double* A, size_t rs, size_t cs,
                 double2 cw = *xw;
 #pragma unroll
                 for (int h = 0; h < 2; ++h)
-                    tri_dmma(cw.x, cw.y, dg.d[iw * 33 + 8 * t + (DESC ? 7 - 4 * h - q : 4 * h + q)], b[h]);
+                    tri_dmma(cw.x, cw.y, bd[tri_e(iw, 8 * t + (DESC ? 7 - 4 * h - q : 4 * h + q))], b[h]);
                 *xw = cw;
             }
             __syncwarp();
