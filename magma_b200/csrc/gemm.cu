@@ -601,18 +601,31 @@ static magma_int_t gemm_launch_tc(bool TA, bool TB, const GemmSizes& g, T alpha,
     }
 }
 
-// NN form of the FP64 tensor-core tile fed by the cp.async pipeline of gemm_async_kernel:
-// three K chunks of 16 in flight (element-sized copies, zero-filled past the edges) into
-// rows padded to 68 doubles, the same fragments, k-steps and epilogue as gemm_dmma_kernel,
-// so the same bits.
+// NN form of the FP64 tensor-core tile fed by a cp.async pipeline: three K chunks of 16 in
+// flight, the same fragments, k-steps and epilogue as gemm_dmma_kernel, so the same bits. A is
+// staged by columns (rows padded to 68 doubles), B by its own columns (16 values of k, padded to
+// 20): both copies run along the contiguous direction, 16 bytes at a time where the instance's
+// pointer and leading dimension allow it, and both fragments touch every bank once. What lies
+// outside the instance costs nothing: 8x8 sub-tiles past M or N take no MMA and no copy, k-steps
+// past K neither (a whole 64x64 tile is twice the work of an average C of orders 8..128). C's
+// lines are prefetched to L2 at the start. What bounds it: latency at three 4-warp blocks an SM
+// (four with 128 registers spill, two stages instead of three lose more). 20,000 products, M, N, K
+// in 8..128: 1,407 -> 1,239 us; M, N, K in 65..128 2,907 -> 2,550; 10,000 x 128^3 1,735 -> 1,702.
 #ifndef MB200_DMMA_WARP_N
 #define MB200_DMMA_WARP_N 32
 #endif
-constexpr int kDmmaWarpN = MB200_DMMA_WARP_N;
+constexpr int kDmmaWarpN = MB200_DMMA_WARP_N, kDmmaStages = 3;
 struct GemmDmmaAsyncSmem {
-    double a[3][16][68];
-    double b[3][16][68];
+    double a[kDmmaStages][16][68];   // [stage][k][row]
+    double b[kDmmaStages][64][20];   // [stage][column][k]
 };
+
+// 16 bytes global -> shared, the first `bytes` (0, 8 or 16) of them read, the rest zero.
+__device__ __forceinline__ void cp_async_16(void* dst, const void* src, int bytes) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(static_cast<unsigned>(__cvta_generic_to_shared(dst))),
+                 "l"(src), "r"(bytes)
+                 : "memory");
+}
 
 // WN: each warp's tile is 32 x WN (4 x WN/8 tiles of 8x8); 64 x 64 / (32 WN) warps.
 template <int WN>
@@ -620,8 +633,7 @@ __global__ void __launch_bounds__(64 * 64 / (32 * WN) * 32, (WN == 16 ? 2 : 3))
 gemm_dmma_async_kernel(GemmSizes g, double alpha, const double* const* __restrict__ A_arr,
                        const double* const* __restrict__ B_arr, double beta, double** __restrict__ C_arr,
                        int tiles_m, int tiles_n, WorkList wl) {
-    constexpr int BM = 64, BN = 64, BK = 16, NT = 64 * 64 / (32 * WN) * 32, ST = 3, TJ = WN / 8;
-    constexpr int EA = BM * BK / NT, EB = BK * BN / NT;
+    constexpr int BM = 64, BN = 64, BK = 16, NT = 64 * 64 / (32 * WN) * 32, ST = kDmmaStages, TJ = WN / 8;
     extern __shared__ __align__(16) unsigned char gemm_dmma_async_raw[];
     GemmDmmaAsyncSmem& sm = *reinterpret_cast<GemmDmmaAsyncSmem*>(gemm_dmma_async_raw);
     const int tiles = tiles_m * tiles_n;
@@ -645,41 +657,98 @@ gemm_dmma_async_kernel(GemmSizes g, double alpha, const double* const* __restric
     for (int i = 0; i < 4; ++i)
 #pragma unroll
         for (int j = 0; j < TJ; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+    // rows and columns the tile's live 8x8 sub-tiles cover
+    const int mlive = min(BM, (m - i0 + 7) & ~7), nlive = min(BN, (n - j0 + 7) & ~7);
+    const int ti = max(0, min(4, (mlive - wm) / 8)), tj = max(0, min(TJ, (nlive - wn) / 8));   // the warp's
+    const bool va = ((reinterpret_cast<size_t>(A) | (size_t)lda * 8) & 15) == 0;
+    const bool vb = ((reinterpret_cast<size_t>(B) | (size_t)ldb * 8) & 15) == 0;
     auto issue = [&](int chunk) {
-        const int st = chunk % ST, k0 = chunk * BK;
+        const int st = chunk % ST, k0 = chunk * BK, kl = min(BK, (k - k0 + 3) & ~3);   // live k's of the chunk
+        if (va) {   // two rows at a time
+            const int r = 2 * (tid & 31), left = 8 * max(0, min(2, m - i0 - r));
+            const double* src = A + i0 + r + (size_t)(k0 + (tid >> 5)) * lda;
 #pragma unroll
-        for (int e = 0; e < EA; ++e) {   // A (M x K, column-major): rows fastest, contiguous
-            const int idx = tid + e * NT, r = idx % BM, c = idx / BM;
-            const bool v = (i0 + r < m) && (k0 + c < k);
-            cp_async_elem(&sm.a[st][c][r], v ? A + (i0 + r) + (size_t)(k0 + c) * lda : A, v, 8);
+            for (int e = 0; e < 32 * BK / NT; ++e) {
+                const int c = (tid >> 5) + e * (NT / 32);
+                if (r < mlive && c < kl) cp_async_16(&sm.a[st][c][r], left ? src : A, k0 + c < k ? left : 0);
+                src += (size_t)(NT / 32) * lda;
+            }
+        } else {
+            for (int e = tid; e < 64 * kl; e += NT) {
+                const int r = e & 63, c = e >> 6;
+                if (r < mlive) {
+                    const bool v = (i0 + r < m) && (k0 + c < k);
+                    cp_async_elem(&sm.a[st][c][r], v ? A + (i0 + r) + (size_t)(k0 + c) * lda : A, v, 8);
+                }
+            }
         }
+        if (vb) {   // two k's at a time
+            const int c = 2 * (tid & 7), left = 8 * max(0, min(2, k - k0 - c));
+            const double* src = B + k0 + c + (size_t)(j0 + (tid >> 3)) * ldb;
 #pragma unroll
-        for (int e = 0; e < EB; ++e) {   // B (K x N, column-major): k fastest, contiguous
-            const int idx = tid + e * NT, c = idx % BK, j = idx / BK;
-            const bool v = (k0 + c < k) && (j0 + j < n);
-            cp_async_elem(&sm.b[st][c][j], v ? B + (k0 + c) + (size_t)(j0 + j) * ldb : B, v, 8);
+            for (int e = 0; e < 8 * BN / NT; ++e) {
+                const int j = (tid >> 3) + e * (NT / 8);
+                if (j < nlive && c < kl) cp_async_16(&sm.b[st][j][c], left ? src : B, j0 + j < n ? left : 0);
+                src += (size_t)(NT / 8) * ldb;
+            }
+        } else {
+            for (int e = tid; e < 16 * nlive; e += NT) {
+                const int c = e & 15, j = e >> 4;
+                if (c < kl) {
+                    const bool v = (k0 + c < k) && (j0 + j < n);
+                    cp_async_elem(&sm.b[st][j][c], v ? B + (k0 + c) + (size_t)(j0 + j) * ldb : B, v, 8);
+                }
+            }
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
     const int nchunks = (k + BK - 1) / BK;
     if (nchunks > 0) issue(0);
     if (nchunks > 1) issue(1); else asm volatile("cp.async.commit_group;" ::: "memory");
+    // C is read after the last product: its lines start towards L2 now
+    if (beta != 0.0)
+        for (int e = tid; e < 4 * nlive; e += NT) {
+            const int r = 16 * (e & 3), j = e >> 2;
+            if (i0 + r < m && j0 + j < n)
+                asm volatile("prefetch.global.L2 [%0];" ::"l"(C + (i0 + r) + (size_t)(j0 + j) * ldc));
+        }
     for (int c = 0; c < nchunks; ++c) {
         asm volatile("cp.async.wait_group 1;" ::: "memory");   // chunk c has landed (c+1 may be in flight)
         __syncthreads();                                         // ... for every thread; stage (c+2)%3 is free
         if (c + 2 < nchunks) issue(c + 2); else asm volatile("cp.async.commit_group;" ::: "memory");
-        const int st = c % ST;
+        const int st = c % ST, steps = min(4, (k - c * BK + 3) / 4);
+        if (ti == 4 && tj == TJ) {
 #pragma unroll
-        for (int s4 = 0; s4 < BK / 4; ++s4) {
-            double af[4], bf[TJ];
+            for (int s4 = 0; s4 < BK / 4; ++s4) {
+                if (s4 < steps) {
+                    double af[4], bf[TJ];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) af[i] = sm.a[st][4 * s4 + q][wm + 8 * i + r8];
+                    for (int i = 0; i < 4; ++i) af[i] = sm.a[st][4 * s4 + q][wm + 8 * i + r8];
 #pragma unroll
-            for (int j = 0; j < TJ; ++j) bf[j] = sm.b[st][4 * s4 + q][wn + 8 * j + r8];
+                    for (int j = 0; j < TJ; ++j) bf[j] = sm.b[st][wn + 8 * j + r8][4 * s4 + q];
 #pragma unroll
-            for (int i = 0; i < 4; ++i)
+                    for (int i = 0; i < 4; ++i)
 #pragma unroll
-                for (int j = 0; j < TJ; ++j) gemm_dmma(acc[i][j][0], acc[i][j][1], af[i], bf[j]);
+                        for (int j = 0; j < TJ; ++j) gemm_dmma(acc[i][j][0], acc[i][j][1], af[i], bf[j]);
+                }
+            }
+        } else if (ti > 0 && tj > 0) {   // the tile's edge
+#pragma unroll 1
+            for (int s4 = 0; s4 < steps; ++s4) {
+                double af[4], bf[TJ];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) af[i] = sm.a[st][4 * s4 + q][wm + 8 * i + r8];
+#pragma unroll
+                for (int j = 0; j < TJ; ++j) bf[j] = sm.b[st][wn + 8 * j + r8][4 * s4 + q];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    if (i < ti) {
+#pragma unroll
+                        for (int j = 0; j < TJ; ++j)
+                            if (j < tj) gemm_dmma(acc[i][j][0], acc[i][j][1], af[i], bf[j]);
+                    }
+                }
+            }
         }
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
