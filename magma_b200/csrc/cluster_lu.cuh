@@ -247,6 +247,14 @@ __device__ __forceinline__ int warp_argmax_lane(const PivotKey& key, int p) {
     return __ffs(who) - 1;
 }
 
+// How a pivot scales its column: 0 a zero pivot (not at all), 1 by its reciprocal, 2 by division
+// (below the smallest normal number, or NaN: dgetf2's other branch). From the bits: a comparison
+// in FP64 costs a step's chain as much as two multiplications.
+__device__ __forceinline__ int pivot_kind(double x) {
+    const unsigned h = (unsigned)__double2hiint(x) & 0x7fffffffu;
+    return (h | (unsigned)__double2loint(x)) == 0 ? 0 : h - 0x00100000u <= 0x7ff00000u - 0x00100000u ? 1 : 2;
+}
+
 // Factors panel columns k0 .. k0+nbp-1 of the rows held in `a` (thread t = row t of the
 // cluster): the steps of lu_panel_steps with the pivot chosen across the cluster. The code of
 // CK steps serves every chunk of CK columns: a finished chunk's columns go to U (column c of
@@ -294,9 +302,9 @@ __device__ __forceinline__ void cluster_panel(double (&a)[NB], int m, int nbp, i
                 double2* row2 = reinterpret_cast<double2*>(mine.row);
 #pragma unroll
                 for (int j = jw; j < NB; j += 2) row2[j / 2] = make_double2(a[j], a[j + 1]);
-                const bool zero = d == 0.0;
-                mine.kind = zero ? 0 : fabs(d) < tiny_normal<double>() ? 2 : 1;
-                mine.rcp = 1.0 / (zero ? 1.0 : d);
+                const int kd = pivot_kind(d);
+                mine.kind = kd;
+                mine.rcp = 1.0 / (kd ? d : 1.0);
                 if constexpr (CS > 1) {
                     mine.hi = key.hi;
                     mine.lo = key.lo;

@@ -17,7 +17,11 @@ namespace mb200 {
 // MPB matrices per block when NW == 1 (one warp each); one matrix per block otherwise.
 template <int NW> struct BlockShape { static constexpr int MPB = (NW == 1) ? 4 : 1; };
 // Blocks per SM the register budget is sized for (<= 128 registers a thread for NC <= 32).
-template <int NC, int NW> struct MinBlocks { static constexpr int value = (NC <= 32 && NW == 1) ? 3 : 1; };
+// getrf alone of 32 columns gains with four (10,000 x 32^2: 104 -> 95 us); gesv and getrs lose
+// (186 -> 195).
+template <int NC, int NW> struct MinBlocks {
+    static constexpr int value = (NC <= 32 && NW == 1) ? 3 : 1, factor = (NC == 32 && NW == 1) ? 4 : value;
+};
 
 template <typename T, int NC, int NW>
 __device__ __forceinline__ void load_rows(T (&a)[NC], const T* __restrict__ A, int m, int n, int lda, int tid) {
@@ -101,7 +105,7 @@ __device__ __forceinline__ void gesv_small_instance(int id, const LuSizes& sz, T
 // ---------------------------------------------------------------------------
 // getrf
 template <typename T, int NC, int NW>
-__global__ void __launch_bounds__(32 * NW * BlockShape<NW>::MPB, MinBlocks<NC, NW>::value)
+__global__ void __launch_bounds__(32 * NW * BlockShape<NW>::MPB, MinBlocks<NC, NW>::factor)
 getrf_small_kernel(WorkList wl, LuSizes sz, T** dA_array, int** ipiv_array, int* info_array) {
     constexpr int MPB = BlockShape<NW>::MPB;
     __shared__ SmallLuShared<T, NC, NW> shm[MPB];

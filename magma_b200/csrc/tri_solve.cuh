@@ -23,6 +23,7 @@
 // 3,963 -> 493.
 #pragma once
 
+#include "fast_div.cuh"
 #include "small_lu.cuh"
 
 namespace mb200 {
@@ -58,36 +59,6 @@ __device__ __forceinline__ void tri_dmma(double& d0, double& d1, double a, doubl
         : "+d"(d0), "+d"(d1)
         : "d"(a), "d"(b));
 }
-
-// A diagonal entry prepared for div_fast: d, the rounded reciprocal and its error term.
-struct TriDivisor {
-    double d, hi, lo;
-};
-__device__ __forceinline__ TriDivisor tri_divisor(double d) {
-    const double r = 1.0 / d;
-    return {d, r, fma_rn(-d, r, 1.0) * r};
-}
-// Operands for which div_fast's products neither overflow nor lose bits: a zero or in
-// 2^-700 .. 2^700, d in 2^-250 .. 2^250.
-__device__ __forceinline__ bool div_fast_num(double a) {
-    const unsigned h = (unsigned)__double2hiint(a) & 0x7fffffffu;
-    return h - (323u << 20) < (1400u << 20) || (h | (unsigned)__double2loint(a)) == 0;
-}
-__device__ __forceinline__ bool div_fast_den(double d) {
-    return ((unsigned)__double2hiint(d) & 0x7fffffffu) - (773u << 20) < (500u << 20);
-}
-// a / d, correctly rounded (Markstein, "Computation of elementary functions on the IBM RISC
-// System/6000 processor", 1990: for q within one ulp of a / d, the exact residual r = a - d q
-// and rd the rounded reciprocal, q + r rd rounds to the quotient). a (hi + lo) rounds to within
-// one ulp. Four operations on the chain of a substitution step; a division is about 130 cycles.
-// A zero a keeps its sign through a * hi.
-__device__ __forceinline__ double div_fast(double a, const TriDivisor& v) {
-    const double q = fma_rn(a, v.hi, a * v.lo);
-    const double x = fma_rn(fma_rn(-v.d, q, a), v.hi, q);
-    return (((unsigned)__double2hiint(a) & 0x7fffffffu) | (unsigned)__double2loint(a)) == 0 ? a * v.hi : x;
-}
-// The division itself, for the operands div_fast does not take; kept out of the unrolled steps.
-static __device__ __noinline__ double div_slow(double a, double d) { return a / d; }
 
 // One sweep of a team of NW >= 2 warps (team.sync() is its barrier). T(i, k) = A[i * rs + k * cs];
 // lower and ascending, or upper and descending (DESC). X holds ceil(n / 32) * 32 rows. On entry
@@ -147,10 +118,10 @@ __device__ __forceinline__ void tri_sweep(const double* A, size_t rs, size_t cs,
             double l[8];
 #pragma unroll
             for (int k = 0; k < 8; ++k) l[k] = bd[tri_e(i, 8 * t + k)];
-            TriDivisor v;
+            Divisor v;
             bool slow = false;   // a diagonal entry of the piece that div_fast cannot take
             if constexpr (MODE != TriDiag::Unit) {
-                v = tri_divisor(j0 + i < n ? bd[tri_e(i, i)] : 1.0);
+                v = make_divisor(j0 + i < n ? bd[tri_e(i, i)] : 1.0);
                 if (MODE == TriDiag::Divide) slow = __any_sync(kFullMask, !div_fast_den(v.d));
             }
 #pragma unroll
