@@ -70,7 +70,10 @@ def ptr_array(t: torch.Tensor) -> torch.Tensor:
         raise ValueError("ptr_array needs a CUDA tensor (the library takes device pointer arrays)")
     n = t.shape[0]
     step = t.stride(0) * t.element_size()
-    return t.data_ptr() + torch.arange(n, device=t.device, dtype=torch.int64) * step
+    p = t.data_ptr()
+    if n > 0 and step > 0:   # one launch: a small batch's call is made of launches
+        return torch.arange(p, p + n * step, step, device=t.device, dtype=torch.int64)
+    return p + torch.arange(n, device=t.device, dtype=torch.int64) * step
 
 
 def _vp(t: torch.Tensor | None) -> C.c_void_p:
