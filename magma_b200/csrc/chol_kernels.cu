@@ -70,10 +70,10 @@ potrs_blocked_kernel(WorkList wl, LuSizes sz, bool upper, T** dA_array, T** dB_a
     }
 }
 
-// ---- FP64 potrf (n <= S) / potrs (n <= ROWS) by a block of S threads ----
-template <int S>
-__global__ void __launch_bounds__(S, (S <= 128 ? 4 : S == 256 ? 2 : 1))
-potrf_team_kernel(WorkList wl, LuSizes sz, bool upper, double** dA_array, int* info_array) {
+// ---- potrf (n <= S) and FP64 potrs (n <= ROWS) by a block of S threads ----
+template <typename T, int S>
+__global__ void __launch_bounds__(S, (sizeof(T) == 4 ? (S == 512 ? 2 : 768 / S) : S <= 128 ? 4 : S == 256 ? 2 : 1))
+potrf_team_kernel(WorkList wl, LuSizes sz, bool upper, T** dA_array, int* info_array) {
     const BlockTeam team;
     for (int w = blockIdx.x; w < wl.size(); w += gridDim.x) {
         const int id = wl.at(w), n = sz.get_n(id);
@@ -147,9 +147,9 @@ static void launch_potrs_small(const WorkList& wl, int bound, bool persistent, c
 template <typename T, int NB, int NT, int CW, int CB>
 static void launch_potrf_blocked(const WorkList& wl, int bound, bool persistent, const LuSizes& sz, bool upper,
                                  T** A, int* info, cudaStream_t s) {
-    if constexpr (std::is_same<T, double>::value && NT <= 512) {
-        auto k = potrf_team_kernel<NT>;
-        const int smem = (int)chol_team_smem(NT);
+    if constexpr (NT <= 512) {
+        auto k = potrf_team_kernel<T, NT>;
+        const int smem = (int)(sizeof(T) == 8 ? chol_team_smem(NT) : sizeof(T) * (32 * NT + 32 * 33 + 32) + 16);
         ensure_dynamic_smem((const void*)k, smem);
         k<<<grid_for(k, NT, bound, persistent, smem), NT, smem, s>>>(wl, sz, upper, A, info);
         return;

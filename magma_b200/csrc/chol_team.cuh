@@ -1,4 +1,4 @@
-// chol_team.cuh -- blocked FP64 Cholesky (potrf) and solve (potrs) of one matrix by a team of
+// chol_team.cuh -- blocked Cholesky (potrf; FP64 or FP32) and FP64 solve (potrs) of one matrix by a team of
 // warps (a thread block, or a range of warps of the one-launch kernel), n <= the team's threads.
 //
 //   for each panel of 32 columns (k0 = 0, 32, ...):
@@ -18,6 +18,9 @@
 // every row stepping through the panel and a row-per-thread solve (one launch for all orders,
 // 8 RHS): 2,000 x 128^2 posv 885 -> 590 us, 740 x 256^2 1,418 -> 827, 444 x 512^2 4,099 -> 2,250;
 // 50,000 orders 4..512 13.6 -> 8.6 ms.
+//
+// FP32 (the mixed solve's factor) runs the same code with FP32 arithmetic, its updates as fma's on
+// the CUDA cores: a warp takes 16 rows x 64 columns there too, 4 x 8 a lane.
 //
 // Per element the operations are those of chol_panel_steps: l(i,k) = a(i,k) * (1 / sqrt(d_k)),
 // a(i,j) = fma(-l(i,k), l(j,k), a(i,j)) for ascending k, so factors, solutions and info are
@@ -40,6 +43,10 @@ constexpr size_t chol_team_smem(int S) {
 // Column c of P's row i sits at P[c * S + (i ^ chol_swz(c))] (see tri_e).
 __device__ __forceinline__ int chol_swz(int c) { return ((c & 3) << 2) | ((c >> 2) & 3); }
 
+// Row i's place in column c of P: swizzled for the FP64 fragments, plain for FP32's vectors.
+template <typename T>
+__device__ __forceinline__ int chol_pos(int i, int c) { return sizeof(T) == 8 ? i ^ chol_swz(c) : i; }
+
 // Warp 0: factors the nbp x nbp diagonal block whose row `lane` is in `a` (zero past nbp), writes
 // it to A (at element (i, j) = A + i si + j sj), L11^T to Lt (row k at Lt + 32 k) and
 // 1 / L11(k,k) to rc. Returns the failing step or -1. The steps run in chunks of eight (one code,
@@ -48,21 +55,23 @@ __device__ __forceinline__ int chol_swz(int c) { return ((c & 3) << 2) | ((c >> 
 // step's chain is the square root, the reciprocal, two products and a shuffle. No step branches:
 // a row's entries right of its diagonal hold values that nothing reads, and from a failing pivot on
 // the multipliers are zero.
-__device__ __forceinline__ int chol_team_diag(double (&a)[32], double* __restrict__ A, size_t si, size_t sj, int nbp,
-                                              double* Lt, double* rc, int lane) {
+template <typename T>
+__device__ __forceinline__ int chol_team_diag(T (&a)[32], T* __restrict__ A, size_t si, size_t sj, int nbp, T* Lt,
+                                              T* rc, int lane) {
+    using V2 = typename Vec2<T>::type;
     int stop = 32;   // first step whose pivot is not positive (the zero padding's, past nbp, too)
 #pragma unroll 1
     for (int c0 = 0; c0 < nbp; c0 += 8) {
-        double l[8];
-        double d = __shfl_sync(kFullMask, a[0], c0);
+        T l[8];
+        T d = __shfl_sync(kFullMask, a[0], c0);
         static_for<0, 8>([&](auto kc) {
             constexpr int k = decltype(kc)::value;
             const int g = c0 + k;
-            if (!(d > 0.0)) stop = min(stop, g);   // not positive definite, or NaN: A(g,g) keeps d
+            if (!(d > T(0))) stop = min(stop, g);   // not positive definite, or NaN: A(g,g) keeps d
             const bool ok = g < stop;
-            const double s = sqrt_rn(ok ? d : 1.0);
-            const double r = 1.0 / s;
-            l[k] = ok ? a[k] * r : 0.0;
+            const T s = sqrt_rn(ok ? d : T(1));
+            const T r = T(1) / s;
+            l[k] = ok ? a[k] * r : T(0);
             // the next pivot needs its own row's multiplier alone
             if constexpr (k < 7) d = __shfl_sync(kFullMask, fma_rn(-l[k], l[k], a[k + 1]), g + 1);
             if (ok) a[k] = lane == g ? s : l[k];
@@ -81,10 +90,10 @@ __device__ __forceinline__ int chol_team_diag(double (&a)[32], double* __restric
             if (jg < 32 - c0) {
 #pragma unroll
                 for (int k = 0; k < 8; ++k) {
-                    const double2* u2 = reinterpret_cast<const double2*>(Lt + 32 * (c0 + k) + c0 + jg);
+                    const V2* u2 = reinterpret_cast<const V2*>(Lt + 32 * (c0 + k) + c0 + jg);
 #pragma unroll
                     for (int j = 0; j < 8; j += 2) {
-                        const double2 u = u2[j / 2];
+                        const V2 u = u2[j / 2];
                         a[jg + j] = fma_rn(-l[k], u.x, a[jg + j]);
                         a[jg + j + 1] = fma_rn(-l[k], u.y, a[jg + j + 1]);
                     }
@@ -99,73 +108,125 @@ __device__ __forceinline__ int chol_team_diag(double (&a)[32], double* __restric
 
 // Dynamic shared memory of the kernel, from byte `off` on (functions that are not inlined take
 // offsets: a pointer argument would lose its address space).
-__device__ __forceinline__ double* chol_smem(unsigned off) {
+template <typename T>
+__device__ __forceinline__ T* chol_smem(unsigned off) {
     extern __shared__ __align__(16) unsigned char chol_team_raw[];
-    return reinterpret_cast<double*>(chol_team_raw + off);
+    return reinterpret_cast<T*>(chol_team_raw + off);
 }
 
 // Warp 0's part of a panel: the diagonal block at k0, first brought up to date with the previous
 // panel's rows (k0 > 0), is factored; *failed (behind rc) gets the failing step or -1. `off`: the
 // team's shared memory (P, then Lt, rc, failed). Not inlined: its registers are its own and its
 // code is in the instruction cache once.
-static __device__ __noinline__ void chol_team_lead(double* A, size_t si, size_t sj, int n, int k0, unsigned off,
+template <typename T>
+__device__ __noinline__ void chol_team_lead(T* A, size_t si, size_t sj, int n, int k0, unsigned off,
                                                    int S) {
-    double* P = chol_smem(off);
-    double* Lt = P + 32 * (size_t)S;
-    double* rc = Lt + 32 * 33;
+    T* P = chol_smem<T>(off);
+    T* Lt = P + 32 * (size_t)S;
+    T* rc = Lt + 32 * 33;
     const int lane = threadIdx.x & 31, q = lane & 3, r8 = lane >> 2;
     const int nbp = min(32, n - k0);
-    double* Ak = A + k0 * si + k0 * sj;
-    double a[32];
-    if (k0 > 0) {
-        // 8x8 tiles of the lower triangle; a lane's A and B fragments are the same entries
-        double c[4][4][2];
-#pragma unroll
-        for (int g = 0; g < 4; ++g)
-#pragma unroll
-            for (int t = 0; t <= g; ++t)
-#pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    const int i = 8 * g + r8, j = 8 * t + 2 * q + h;
-                    c[g][t][h] = (i < nbp && j <= i) ? Ak[i * si + j * sj] : 0.0;
-                }
-#pragma unroll
-        for (int s = 0; s < 8; ++s) {
-            double f[4];
-#pragma unroll
-            for (int g = 0; g < 4; ++g) f[g] = P[(4 * s + q) * S + ((k0 + 8 * g + r8) ^ chol_swz(4 * s + q))];
+    T* Ak = A + k0 * si + k0 * sj;
+    T a[32];
+    if constexpr (std::is_same<T, double>::value) {
+        if (k0 > 0) {
+            // 8x8 tiles of the lower triangle; a lane's A and B fragments are the same entries
+            double c[4][4][2];
 #pragma unroll
             for (int g = 0; g < 4; ++g)
 #pragma unroll
-                for (int t = 0; t <= g; ++t) chol_dmma(c[g][t][0], c[g][t][1], -f[g], f[t]);
+                for (int t = 0; t <= g; ++t)
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        const int i = 8 * g + r8, j = 8 * t + 2 * q + h;
+                        c[g][t][h] = (i < nbp && j <= i) ? Ak[i * si + j * sj] : 0.0;
+                    }
+#pragma unroll
+            for (int s = 0; s < 8; ++s) {
+                double f[4];
+#pragma unroll
+                for (int g = 0; g < 4; ++g) f[g] = P[(4 * s + q) * S + ((k0 + 8 * g + r8) ^ chol_swz(4 * s + q))];
+#pragma unroll
+                for (int g = 0; g < 4; ++g)
+#pragma unroll
+                    for (int t = 0; t <= g; ++t) chol_dmma(c[g][t][0], c[g][t][1], -f[g], f[t]);
+            }
+#pragma unroll
+            for (int g = 0; g < 4; ++g)
+#pragma unroll
+                for (int t = 0; t <= g; ++t)
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) Lt[33 * (8 * g + r8) + 8 * t + 2 * q + h] = c[g][t][h];
+            __syncwarp();
+#pragma unroll
+            for (int j = 0; j < 32; ++j) a[j] = (lane < nbp && j <= lane) ? Lt[33 * lane + j] : 0.0;
+            __syncwarp();
+        } else {
+#pragma unroll
+            for (int j = 0; j < 32; ++j) a[j] = (lane < nbp && j <= lane) ? Ak[lane * si + j * sj] : 0.0;
         }
-#pragma unroll
-        for (int g = 0; g < 4; ++g)
-#pragma unroll
-            for (int t = 0; t <= g; ++t)
-#pragma unroll
-                for (int h = 0; h < 2; ++h) Lt[33 * (8 * g + r8) + 8 * t + 2 * q + h] = c[g][t][h];
-        __syncwarp();
-#pragma unroll
-        for (int j = 0; j < 32; ++j) a[j] = (lane < nbp && j <= lane) ? Lt[33 * lane + j] : 0.0;
-        __syncwarp();
     } else {
 #pragma unroll
-        for (int j = 0; j < 32; ++j) a[j] = (lane < nbp && j <= lane) ? Ak[lane * si + j * sj] : 0.0;
+        for (int j = 0; j < 32; ++j) a[j] = (lane < nbp && j <= lane) ? Ak[lane * si + j * sj] : T(0);
+        if (k0 > 0) {
+#pragma unroll 2
+            for (int c = 0; c < 32; ++c) {   // lane = row; the block's own columns are broadcast
+                const T* Pc = P + c * S + k0;
+                const T l = Pc[lane];
+#pragma unroll
+                for (int j = 0; j < 32; j += 4) {
+                    const float4 u = *reinterpret_cast<const float4*>(Pc + j);
+                    a[j] = fma_rn(-l, u.x, a[j]);
+                    a[j + 1] = fma_rn(-l, u.y, a[j + 1]);
+                    a[j + 2] = fma_rn(-l, u.z, a[j + 2]);
+                    a[j + 3] = fma_rn(-l, u.w, a[j + 3]);
+                }
+            }
+        }
     }
     const int f = chol_team_diag(a, Ak, si, sj, nbp, Lt, rc, lane);
     if (lane == 0) *reinterpret_cast<int*>(rc + 32) = f;
     __syncwarp();
 }
 
+// FP32 trailing update of 16 rows from i0 on, columns jb .. je: lane = 4 rows x 8 columns.
+__device__ __forceinline__ void chol_team_update(float* __restrict__ A, int n, size_t si, size_t sj, int i0, int jb,
+                                                 int je, const float* P, int S, int lane) {
+    const int i = i0 + 4 * (lane & 3), j = jb + 8 * (lane >> 2);
+    if (j >= je) return;
+    float acc[4][8];
+#pragma unroll
+    for (int c = 0; c < 8; ++c)
+#pragma unroll
+        for (int r = 0; r < 4; ++r)
+            acc[r][c] = (i + r < n && j + c <= i + r) ? A[(i + r) * si + (j + c) * sj] : 0.0f;
+#pragma unroll 4
+    for (int k = 0; k < 32; ++k) {
+        const float4 l = *reinterpret_cast<const float4*>(P + k * S + i);
+        const float4 u = *reinterpret_cast<const float4*>(P + k * S + j);
+        const float4 v = *reinterpret_cast<const float4*>(P + k * S + j + 4);
+        const float lr[4] = {l.x, l.y, l.z, l.w}, uc[8] = {u.x, u.y, u.z, u.w, v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int r = 0; r < 4; ++r)
+#pragma unroll
+            for (int c = 0; c < 8; ++c) acc[r][c] = fma_rn(-lr[r], uc[c], acc[r][c]);
+    }
+#pragma unroll
+    for (int c = 0; c < 8; ++c)
+#pragma unroll
+        for (int r = 0; r < 4; ++r)
+            if (i + r < n && j + c <= i + r) A[(i + r) * si + (j + c) * sj] = acc[r][c];
+}
+
 // potrf of one n x n matrix (n <= S) by the team's S threads; `off`: its shared memory. Returns
 // info; the caller synchronises the team before it reuses the shared memory.
-template <typename Team>
-__device__ int chol_team_potrf(double* __restrict__ A, int n, int lda, bool upper, unsigned off, int S,
+template <typename T, typename Team>
+__device__ int chol_team_potrf(T* __restrict__ A, int n, int lda, bool upper, unsigned off, int S,
                                const Team& team) {
-    double* P = chol_smem(off);
-    double* Lt = P + 32 * (size_t)S;   // the updated diagonal block (row i at 33 i), then L11^T
-    double* rc = Lt + 32 * 33;
+    using V2 = typename Vec2<T>::type;
+    T* P = chol_smem<T>(off);
+    T* Lt = P + 32 * (size_t)S;   // the updated diagonal block (row i at 33 i), then L11^T
+    T* rc = Lt + 32 * 33;
     int* failed = reinterpret_cast<int*>(rc + 32);
     const int tid = team.tid(), lane = tid & 31, warp = tid >> 5, NW = S >> 5;
     const int q = lane & 3, r8 = lane >> 2;
@@ -177,19 +238,19 @@ __device__ int chol_team_potrf(double* __restrict__ A, int n, int lda, bool uppe
         const int m0 = k0 + 32, fail = *failed, steps = fail >= 0 ? fail : 32;
         // ---- rows below the diagonal block ----
         if (tid >= m0 && tid < n) {
-            double a[32];
-            double* row = A + tid * si + k0 * sj;
+            T a[32];
+            T* row = A + tid * si + k0 * sj;
 #pragma unroll
             for (int c = 0; c < 32; ++c) a[c] = row[c * sj];
             static_for<0, 32>([&](auto kc) {
                 constexpr int k = decltype(kc)::value;
                 if (k < steps) {
-                    const double l = a[k] * rc[k];
+                    const T l = a[k] * rc[k];
                     a[k] = l;
-                    const double2* u2 = reinterpret_cast<const double2*>(Lt + 32 * k);
+                    const V2* u2 = reinterpret_cast<const V2*>(Lt + 32 * k);
 #pragma unroll
                     for (int j = (k + 1) & ~1; j < 32; j += 2) {
-                        const double2 u = u2[j / 2];
+                        const V2 u = u2[j / 2];
                         if (j > k) a[j] = fma_rn(-l, u.x, a[j]);
                         a[j + 1] = fma_rn(-l, u.y, a[j + 1]);
                     }
@@ -198,7 +259,7 @@ __device__ int chol_team_potrf(double* __restrict__ A, int n, int lda, bool uppe
 #pragma unroll
             for (int c = 0; c < 32; ++c) {
                 row[c * sj] = a[c];
-                P[c * S + (tid ^ chol_swz(c))] = a[c];
+                P[c * S + chol_pos<T>(tid, c)] = a[c];
             }
         }
         if (fail >= 0) return k0 + fail + 1;
@@ -214,52 +275,57 @@ __device__ int chol_team_potrf(double* __restrict__ A, int n, int lda, bool uppe
                 for (int jb = m0; jb < i0 + 16; jb += 64) {
                     if (turn-- > 0) continue;
                     turn = NW - 2;
-                    const int ra = i0 + r8, rb = ra + 8, je = min(jb + 64, i0 + 16);
-                    double cn[2][2][2];   // [tile][row group][column]
-                    auto load_c = [&](int jt) {
+                    if constexpr (!std::is_same<T, double>::value) {
+                        chol_team_update(A, n, si, sj, i0, jb, min(jb + 64, i0 + 16), P, S, lane);
+                        continue;
+                    } else {
+                        const int ra = i0 + r8, rb = ra + 8, je = min(jb + 64, i0 + 16);
+                        double cn[2][2][2];   // [tile][row group][column]
+                        auto load_c = [&](int jt) {
 #pragma unroll
-                        for (int t = 0; t < 2; ++t)
+                            for (int t = 0; t < 2; ++t)
 #pragma unroll
-                            for (int h = 0; h < 2; ++h) {
-                                const int j = jt + 8 * t + 2 * q + h;
-                                cn[t][0][h] = (ra < n && j <= ra) ? A[ra * si + j * sj] : 0.0;
-                                cn[t][1][h] = (rb < n && j <= rb) ? A[rb * si + j * sj] : 0.0;
-                            }
-                    };
-                    load_c(jb);
-                    double fa[8], fb[8];
-#pragma unroll
-                    for (int s = 0; s < 8; ++s) {
-                        const int c = 4 * s + q;
-                        fa[s] = -P[c * S + (ra ^ chol_swz(c))];
-                        fb[s] = -P[c * S + (rb ^ chol_swz(c))];
-                    }
-#pragma unroll 1
-                    for (int jt = jb; jt < je; jt += 16) {
-                        double cc[2][2][2];
-#pragma unroll
-                        for (int t = 0; t < 2; ++t)
-#pragma unroll
-                            for (int g = 0; g < 2; ++g) { cc[t][g][0] = cn[t][g][0]; cc[t][g][1] = cn[t][g][1]; }
-                        if (jt + 16 < je) load_c(jt + 16);
+                                for (int h = 0; h < 2; ++h) {
+                                    const int j = jt + 8 * t + 2 * q + h;
+                                    cn[t][0][h] = (ra < n && j <= ra) ? A[ra * si + j * sj] : 0.0;
+                                    cn[t][1][h] = (rb < n && j <= rb) ? A[rb * si + j * sj] : 0.0;
+                                }
+                        };
+                        load_c(jb);
+                        double fa[8], fb[8];
 #pragma unroll
                         for (int s = 0; s < 8; ++s) {
                             const int c = 4 * s + q;
-                            const double b0 = P[c * S + ((jt + r8) ^ chol_swz(c))];
-                            const double b1 = P[c * S + ((jt + 8 + r8) ^ chol_swz(c))];
-                            chol_dmma(cc[0][0][0], cc[0][0][1], fa[s], b0);
-                            chol_dmma(cc[0][1][0], cc[0][1][1], fb[s], b0);
-                            chol_dmma(cc[1][0][0], cc[1][0][1], fa[s], b1);
-                            chol_dmma(cc[1][1][0], cc[1][1][1], fb[s], b1);
+                            fa[s] = -P[c * S + (ra ^ chol_swz(c))];
+                            fb[s] = -P[c * S + (rb ^ chol_swz(c))];
                         }
+#pragma unroll 1
+                        for (int jt = jb; jt < je; jt += 16) {
+                            double cc[2][2][2];
 #pragma unroll
-                        for (int t = 0; t < 2; ++t)
+                            for (int t = 0; t < 2; ++t)
 #pragma unroll
-                            for (int h = 0; h < 2; ++h) {
-                                const int j = jt + 8 * t + 2 * q + h;
-                                if (ra < n && j <= ra) A[ra * si + j * sj] = cc[t][0][h];
-                                if (rb < n && j <= rb) A[rb * si + j * sj] = cc[t][1][h];
+                                for (int g = 0; g < 2; ++g) { cc[t][g][0] = cn[t][g][0]; cc[t][g][1] = cn[t][g][1]; }
+                            if (jt + 16 < je) load_c(jt + 16);
+#pragma unroll
+                            for (int s = 0; s < 8; ++s) {
+                                const int c = 4 * s + q;
+                                const double b0 = P[c * S + ((jt + r8) ^ chol_swz(c))];
+                                const double b1 = P[c * S + ((jt + 8 + r8) ^ chol_swz(c))];
+                                chol_dmma(cc[0][0][0], cc[0][0][1], fa[s], b0);
+                                chol_dmma(cc[0][1][0], cc[0][1][1], fb[s], b0);
+                                chol_dmma(cc[1][0][0], cc[1][0][1], fa[s], b1);
+                                chol_dmma(cc[1][1][0], cc[1][1][1], fb[s], b1);
                             }
+#pragma unroll
+                            for (int t = 0; t < 2; ++t)
+#pragma unroll
+                                for (int h = 0; h < 2; ++h) {
+                                    const int j = jt + 8 * t + 2 * q + h;
+                                    if (ra < n && j <= ra) A[ra * si + j * sj] = cc[t][0][h];
+                                    if (rb < n && j <= rb) A[rb * si + j * sj] = cc[t][1][h];
+                                }
+                        }
                     }
                 }
             }
@@ -272,7 +338,7 @@ __device__ int chol_team_potrf(double* __restrict__ A, int n, int lda, bool uppe
 template <typename Team>
 __device__ void chol_team_potrs(const double* A, int n, int lda, bool upper, double* __restrict__ B, int nrhs, int ldb,
                                 unsigned off, int S, int rows, int first, int stride, const Team& team) {
-    double* X = chol_smem(off);
+    double* X = chol_smem<double>(off);
     TriStage& st = *reinterpret_cast<TriStage*>(X + (size_t)rows * kTriRhs);
     const int NW = S >> 5, npad = (n + 31) / 32 * 32;
     const size_t si = upper ? (size_t)lda : 1, sj = upper ? 1 : (size_t)lda;

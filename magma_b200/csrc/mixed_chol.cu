@@ -21,7 +21,7 @@
 #include "internal.h"
 #include "chol_launch.h"
 #include "tuning.h"
-#include "small_lu.cuh"
+#include "tri_solve.cuh"
 #include "vbatched.h"
 #include <algorithm>
 #include <cfloat>
@@ -55,19 +55,35 @@ dlat2s_norm_vkernel(WorkList wl, const int* n_arr, double** dA_array, const int*
         float* SA = dS_array[id];
         bool overflow = false;
         double rowpart = 0.0;
-        if (t < n) {
-            for (int j = 0; j <= t; ++j) {
-                const double a = A[t + (size_t)j * lda];
-                rowpart += fabs(a);
-                overflow |= !(fabs(a) <= (double)FLT_MAX);
-                SA[t + (size_t)j * n] = (float)a;
+        // eight loads before their stores (interleaved, each load would wait for the store before it)
+        for (int j0 = 0; j0 <= (t | 31) && j0 < n; j0 += 8) {
+            double v[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) v[u] = (t < n && j0 + u <= t) ? A[t + (size_t)(j0 + u) * lda] : 0.0;
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                if (t < n && j0 + u <= t) {
+                    rowpart += fabs(v[u]);
+                    overflow |= !(fabs(v[u]) <= (double)FLT_MAX);
+                    SA[t + (size_t)(j0 + u) * n] = (float)v[u];
+                }
             }
         }
-        for (int c = w; c < n; c += NT / 32) {
-            double s = 0.0;
-            for (int k = c + 1 + lane; k < n; k += 32) s += fabs(A[k + (size_t)c * lda]);
-            for (int off = 16; off > 0; off >>= 1) s += __shfl_xor_sync(kFullMask, s, off);
-            if (lane == 0) colpart[c] = s;
+        // four columns a warp at a time
+        for (int c0 = 4 * w; c0 < n; c0 += 4 * (NT / 32)) {
+            double s[4] = {0.0, 0.0, 0.0, 0.0};
+            for (int k = (c0 & ~31) + lane; k < n; k += 32) {
+#pragma unroll
+                for (int u = 0; u < 4; ++u) s[u] += k > c0 + u ? fabs(A[k + (size_t)(c0 + u) * lda]) : 0.0;
+            }
+#pragma unroll
+            for (int off = 16; off > 0; off >>= 1) {
+#pragma unroll
+                for (int u = 0; u < 4; ++u) s[u] += __shfl_xor_sync(kFullMask, s[u], off);
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                if (lane == 0 && c0 + u < n) colpart[c0 + u] = s[u];
         }
         __syncthreads();
         double rs = (t < n) ? rowpart + colpart[t] : 0.0;
@@ -86,115 +102,71 @@ dlat2s_norm_vkernel(WorkList wl, const int* n_arr, double** dA_array, const int*
     }
 }
 
-// ---- 2. refinement: one block per instance, thread t = row t, NT >= n ----
-template <int NT, int R>
+// ---- 2. refinement: one block of NT threads per instance, n <= NMAX, eight right-hand sides at a
+// time. The correction solves L L^T c = r with the FP32 factor on the FP64 tensor cores
+// (tri_solve.cuh), the residual B - A X is a tensor-core product over the stored triangle (a warp
+// per 16 rows). Both read A and L along their contiguous direction whichever triangle an element
+// lies in; the former thread-per-row loops read half of each with 32 lines a load.
+template <int NMAX>
 struct CholRefineSmem {
-    static constexpr int NBLK = NT / 32;
-    float  inv[NBLK][32][33];      // L_JJ^-1 of each 32x32 diagonal block
-    float  sx[2][32][R];           // solved values of the current block (double-buffered)
-    float  sb[NBLK][32][R];        // per-warp staging of a block's right-hand sides
-    double xs[NT][R];              // FP64 solution, shared for the residual
-    double red[2][NBLK][R];
+    double X[NMAX * kTriRhs];      // solution
+    double W[NMAX * kTriRhs];      // residual, then correction
+    double red[2][16][kTriRhs];
+    TriStageOf<float> st;          // orders up to 32 use st.d[0] alone
+    static constexpr size_t bytes() {
+        return sizeof(CholRefineSmem) - (NMAX <= 32 ? 3 * sizeof(float) * 1024 : 0);
+    }
 };
 
-// L_JJ^-1 (lower, non-unit) of diagonal block J of SA, by warp J: lane j forms column j.
-template <int NT, int R>
-__device__ __forceinline__ void chol_invert_diag_block(const float* __restrict__ SA, int n, int J, int lane,
-                                                       CholRefineSmem<NT, R>& sh) {
-    const int j0 = J * 32;
-    float (&T)[32][33] = sh.inv[J];
-#pragma unroll 4
-    for (int k = 0; k < 32; ++k)
-        T[lane][k] = (j0 + lane < n && j0 + k < n) ? (k <= lane ? SA[j0 + lane + (size_t)(j0 + k) * n] : 0.0f)
-                                                   : (lane == k ? 1.0f : 0.0f);
-    __syncwarp();
-    float x[32];
-    static_for<0, 32>([&](auto ic) {
-        constexpr int i = decltype(ic)::value;
-        float s = (i == lane) ? 1.0f : 0.0f;
+// W -= A X, A symmetric with its lower triangle stored; W and X hold npad >= n rows (zero past n).
+template <int NT>
+__device__ __forceinline__ void chol_residual(const double* __restrict__ A, int n, int lda, const double* X, double* W) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, q = lane & 3, r8 = lane >> 2;
+    for (int i0 = 16 * warp; i0 < n; i0 += 16 * (NT / 32)) {
+        const int ia = i0 + r8, ib = ia + 8;
+        double2 c0 = *reinterpret_cast<const double2*>(&W[tri_x(ia, 2 * q)]);
+        double2 c1 = *reinterpret_cast<const double2*>(&W[tri_x(ib, 2 * q)]);
+        double2 e0 = make_double2(0.0, 0.0), e1 = e0;   // odd k-steps
+        double va[8], vb[8];
+        auto load = [&](int k0) {
 #pragma unroll
-        for (int k = 0; k < i; ++k) s = fmaf(-T[i][k], x[k], s);
-        x[i] = (i < lane) ? 0.0f : s / T[i][i];
-    });
-    __syncwarp();
+            for (int s = 0; s < 8; ++s) {
+                const int k = k0 + 4 * s + q;
+                va[s] = (ia < n && k < n) ? (k <= ia ? A[ia + (size_t)k * lda] : A[k + (size_t)ia * lda]) : 0.0;
+                vb[s] = (ib < n && k < n) ? (k <= ib ? A[ib + (size_t)k * lda] : A[k + (size_t)ib * lda]) : 0.0;
+            }
+        };
+        load(0);
+        for (int k0 = 0; k0 < n; k0 += 32) {
+            double ua[8], ub[8];
 #pragma unroll
-    for (int i = 0; i < 32; ++i) T[i][lane] = x[i];
-    __syncwarp();
-}
-
-// L L^T c = b in single precision for the R right-hand sides in f (thread t = row t).
-template <int NT, int R>
-__device__ __forceinline__ void chol_refine_solve(const float* __restrict__ SA, int n, float (&f)[R],
-                                                  CholRefineSmem<NT, R>& sh) {
-    const int t = threadIdx.x, lane = t & 31, w = t >> 5;
-    const int nblk = (n + 31) / 32;
-    auto diag_step = [&](int J, bool transposed, int buf) {
+            for (int s = 0; s < 8; ++s) { ua[s] = va[s]; ub[s] = vb[s]; }
+            if (k0 + 32 < n) load(k0 + 32);
 #pragma unroll
-        for (int r = 0; r < R; ++r) sh.sb[w][lane][r] = f[r];
-        __syncwarp();
-        float x[R];
-#pragma unroll
-        for (int r = 0; r < R; ++r) x[r] = 0.0f;
-#pragma unroll 8
-        for (int k = 0; k < 32; ++k) {
-            const float l = transposed ? sh.inv[J][k][lane] : sh.inv[J][lane][k];
-#pragma unroll
-            for (int r = 0; r < R; ++r) x[r] = fmaf(l, sh.sb[w][k][r], x[r]);
-        }
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-            f[r] = x[r];
-            sh.sx[buf][lane][r] = x[r];
-        }
-    };
-    // forward: L y = b, blocks ascending; rows below take L(i, block) * y_block
-    for (int J = 0; J < nblk; ++J) {
-        const int j0 = J * 32, buf = J & 1;
-        float lv[32];
-        const bool below = (w > J && t < n);
-        if (below) {
-#pragma unroll
-            for (int k = 0; k < 32; ++k) lv[k] = (j0 + k < n) ? SA[t + (size_t)(j0 + k) * n] : 0.0f;
-        }
-        if (w == J) diag_step(J, false, buf);
-        __syncthreads();
-        if (below) {
-#pragma unroll
-            for (int k = 0; k < 32; ++k) {
-#pragma unroll
-                for (int r = 0; r < R; ++r) f[r] = fmaf(-lv[k], sh.sx[buf][k][r], f[r]);
+            for (int s = 0; s < 8; s += 2) {
+                const double b0 = -X[tri_x(k0 + 4 * s + q, r8)], b1 = -X[tri_x(k0 + 4 * s + 4 + q, r8)];
+                tri_dmma(c0.x, c0.y, ua[s], b0);
+                tri_dmma(c1.x, c1.y, ub[s], b0);
+                tri_dmma(e0.x, e0.y, ua[s + 1], b1);
+                tri_dmma(e1.x, e1.y, ub[s + 1], b1);
             }
         }
-    }
-    // backward: L^T x = y, blocks descending; rows above take L(block, i)^T * x_block
-    for (int J = nblk - 1; J >= 0; --J) {
-        const int j0 = J * 32, buf = (2 * nblk - 1 - J) & 1;
-        float uv[32];
-        const bool above = (w < J);
-        if (above) {
-#pragma unroll
-            for (int k = 0; k < 32; ++k) uv[k] = (j0 + k < n) ? SA[j0 + k + (size_t)t * n] : 0.0f;
-        }
-        if (w == J) diag_step(J, true, buf);
-        __syncthreads();
-        if (above) {
-#pragma unroll
-            for (int k = 0; k < 32; ++k) {
-#pragma unroll
-                for (int r = 0; r < R; ++r) f[r] = fmaf(-uv[k], sh.sx[buf][k][r], f[r]);
-            }
-        }
+        *reinterpret_cast<double2*>(&W[tri_x(ia, 2 * q)]) = make_double2(c0.x + e0.x, c0.y + e0.y);
+        *reinterpret_cast<double2*>(&W[tri_x(ib, 2 * q)]) = make_double2(c1.x + e1.x, c1.y + e1.y);
     }
 }
 
-template <int NT, int R>
-__global__ void __launch_bounds__(NT, (NT >= 512 ? 1 : 512 / NT))
+template <int NMAX, int NT>
+__global__ void __launch_bounds__(NT, (NT == 64 ? 8 : NT == 128 ? 4 : 2))
 dsposv_refine_vkernel(WorkList wl, const int* n_arr, const int* nrhs_arr, double** dA_array, const int* ldda,
                       double** dB_array, const int* lddb, double** dX_array, const int* lddx, float** dS_array,
                       CholMixedWs ws, int* iter_array) {
     extern __shared__ __align__(16) unsigned char chol_refine_smem[];
-    CholRefineSmem<NT, R>& sh = *reinterpret_cast<CholRefineSmem<NT, R>*>(chol_refine_smem);
+    CholRefineSmem<NMAX>& sh = *reinterpret_cast<CholRefineSmem<NMAX>*>(chol_refine_smem);
+    constexpr int NW = NT / 32;
+    const BlockTeam team;
     const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+    const int col = t & 7, row0 = t >> 3;        // this thread's right-hand side and first row
     for (int it = blockIdx.x; it < wl.size(); it += gridDim.x) {
         const int id = wl.at(it);
         if (iter_array[id] < 0) continue;        // conversion already failed (block-uniform)
@@ -209,81 +181,54 @@ dsposv_refine_vkernel(WorkList wl, const int* n_arr, const int* nrhs_arr, double
         const int lda = ldda[id], ldb = lddb[id], ldx = lddx[id];
         const float* SA = dS_array[id];
         const double cte = ws.anrm[id] * (DBL_EPSILON * 0.5) * sqrt((double)n);
-        const int nblk = (n + 31) / 32;
-        for (int J = w; J < nblk; J += NT / 32) chol_invert_diag_block<NT, R>(SA, n, J, lane, sh);
-        __syncthreads();
+        const int npad = (n + 31) / 32 * 32;
         int iter_out = 0;
-        for (int c0 = 0; c0 < nrhs && iter_out >= 0; c0 += R) {
-            double b[R], x[R], res[R];
-#pragma unroll
-            for (int r = 0; r < R; ++r) {
-                b[r] = (t < n && c0 + r < nrhs) ? B[t + (size_t)(c0 + r) * ldb] : 0.0;
-                x[r] = 0.0;
-                res[r] = b[r];
+        for (int c0 = 0; c0 < nrhs && iter_out >= 0; c0 += kTriRhs) {
+            const bool live = c0 + col < nrhs;
+            bool ovf = false;
+            for (int i = row0; i < npad; i += NT / 8) {
+                const double b = (i < n && live) ? B[i + (size_t)(c0 + col) * ldb] : 0.0;
+                sh.X[tri_x(i, col)] = 0.0;
+                sh.W[tri_x(i, col)] = b;
+                ovf |= !(fabs(b) <= (double)FLT_MAX);
             }
             int iiter = 0, stalls = 0;
             double prev_ratio = 1e300;
             for (;;) {
-                bool ovf = false;
-                float f[R];
-#pragma unroll
-                for (int r = 0; r < R; ++r) {
-                    ovf |= !(fabs(res[r]) <= (double)FLT_MAX);
-                    f[r] = (float)res[r];
-                }
                 if (__syncthreads_or(ovf)) { iter_out = -2; break; }
-                chol_refine_solve<NT, R>(SA, n, f, sh);
-                if (t < n) {
-#pragma unroll
-                    for (int r = 0; r < R; ++r) {
-                        x[r] += (double)f[r];
-                        sh.xs[t][r] = x[r];
-                    }
+                tri_sweep<TriDiag::Reciprocal, false>(SA, (size_t)1, (size_t)n, n, sh.W, sh.st, NW, team);
+                tri_sweep<TriDiag::Reciprocal, true>(SA, (size_t)n, (size_t)1, n, sh.W, sh.st, NW, team);
+                for (int i = row0; i < npad; i += NT / 8) {
+                    const int e = tri_x(i, col);
+                    sh.X[e] += sh.W[e];
+                    sh.W[e] = (i < n && live) ? B[i + (size_t)(c0 + col) * ldb] : 0.0;
                 }
                 __syncthreads();
-                // R = B - A X with A symmetric, lower triangle stored
-#pragma unroll
-                for (int r = 0; r < R; ++r) res[r] = b[r];
-                if (t < n) {
-#pragma unroll 8
-                    for (int j = 0; j <= t; ++j) {
-                        const double a = A[t + (size_t)j * lda];
-#pragma unroll
-                        for (int r = 0; r < R; ++r) res[r] = fma(-a, sh.xs[j][r], res[r]);
-                    }
-#pragma unroll 8
-                    for (int j = t + 1; j < n; ++j) {
-                        const double a = A[j + (size_t)t * lda];
-#pragma unroll
-                        for (int r = 0; r < R; ++r) res[r] = fma(-a, sh.xs[j][r], res[r]);
-                    }
-                }
-                double xn[R], rn[R];
-#pragma unroll
-                for (int r = 0; r < R; ++r) {
-                    xn[r] = (t < n && c0 + r < nrhs) ? fabs(x[r]) : 0.0;
-                    rn[r] = (t < n && c0 + r < nrhs) ? fabs(res[r]) : 0.0;
-                }
-                // block-wide maxima per right-hand side
-#pragma unroll
-                for (int r = 0; r < R; ++r) {
-                    for (int off = 16; off > 0; off >>= 1) {
-                        xn[r] = fmax(xn[r], __shfl_xor_sync(kFullMask, xn[r], off));
-                        rn[r] = fmax(rn[r], __shfl_xor_sync(kFullMask, rn[r], off));
-                    }
-                }
+                chol_residual<NT>(A, n, lda, sh.X, sh.W);
                 __syncthreads();
-                if (lane == 0) {
-#pragma unroll
-                    for (int r = 0; r < R; ++r) { sh.red[0][w][r] = xn[r]; sh.red[1][w][r] = rn[r]; }
+                double xn = 0.0, rn = 0.0;
+                ovf = false;
+                if (live) {
+                    for (int i = row0; i < n; i += NT / 8) {
+                        const double r = fabs(sh.W[tri_x(i, col)]);
+                        xn = fmax(xn, fabs(sh.X[tri_x(i, col)]));
+                        rn = fmax(rn, r);
+                        ovf |= !(r <= (double)FLT_MAX);
+                    }
                 }
+#pragma unroll
+                for (int off = 8; off < 32; off <<= 1) {   // lanes of one right-hand side
+                    xn = fmax(xn, __shfl_xor_sync(kFullMask, xn, off));
+                    rn = fmax(rn, __shfl_xor_sync(kFullMask, rn, off));
+                }
+                if (lane < 8) { sh.red[0][w][lane] = xn; sh.red[1][w][lane] = rn; }
                 __syncthreads();
                 bool ok = true;
                 double ratio = 0.0;
 #pragma unroll
-                for (int r = 0; r < R; ++r) {
+                for (int r = 0; r < kTriRhs; ++r) {
                     double xm = 0.0, rm = 0.0;
-                    for (int k = 0; k < NT / 32; ++k) { xm = fmax(xm, sh.red[0][k][r]); rm = fmax(rm, sh.red[1][k][r]); }
+                    for (int k = 0; k < NW; ++k) { xm = fmax(xm, sh.red[0][k][r]); rm = fmax(rm, sh.red[1][k][r]); }
                     if (c0 + r < nrhs) {
                         ok &= (rm <= xm * cte);
                         ratio = fmax(ratio, rm / fmax(xm * cte, DBL_MIN));
@@ -297,11 +242,8 @@ dsposv_refine_vkernel(WorkList wl, const int* n_arr, const int* nrhs_arr, double
             }
             if (iter_out < 0) break;
             iter_out = max(iter_out, iiter);
-            if (t < n) {
-#pragma unroll
-                for (int r = 0; r < R; ++r)
-                    if (c0 + r < nrhs) X[t + (size_t)(c0 + r) * ldx] = x[r];
-            }
+            if (live)
+                for (int i = row0; i < n; i += NT / 8) X[i + (size_t)(c0 + col) * ldx] = sh.X[tri_x(i, col)];
             __syncthreads();
         }
         if (t == 0) {
@@ -362,15 +304,15 @@ template <int NT>
 static void launch_bucket_stage(int stage, const WorkList& wl, int batch, const int* n, const int* nrhs, double** A,
                                 const int* lda, double** B, const int* ldb, double** X, const int* ldx, float** S,
                                 const CholMixedWs& ws, int* iter, cudaStream_t s) {
-    constexpr int R = 4;
     if (stage == 0) {
         auto k = dlat2s_norm_vkernel<NT>;
         k<<<persistent_grid(k, NT, 0, batch), NT, 0, s>>>(wl, n, A, lda, S, ws, iter);
     } else {
-        auto k = dsposv_refine_vkernel<NT, R>;
-        const int smem = (int)sizeof(CholRefineSmem<NT, R>);
+        constexpr int RT = NT <= 128 ? 64 : NT / 2;   // refinement threads: two warps up to n = 128
+        auto k = dsposv_refine_vkernel<NT, RT>;
+        const int smem = (int)CholRefineSmem<NT>::bytes();
         ensure_dynamic_smem((const void*)k, smem);
-        k<<<persistent_grid(k, NT, smem, batch), NT, smem, s>>>(wl, n, nrhs, A, lda, B, ldb, X, ldx, S, ws, iter);
+        k<<<persistent_grid(k, RT, smem, batch), RT, smem, s>>>(wl, n, nrhs, A, lda, B, ldb, X, ldx, S, ws, iter);
     }
 }
 

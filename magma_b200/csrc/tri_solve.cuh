@@ -40,17 +40,21 @@ __device__ __forceinline__ int tri_x(int row, int col) { return row * kTriRhs + 
 // The staged blocks of two successive steps: the u-th block in sweep order has its diagonal block
 // in d[u & 1] and the block that couples it to its predecessor in p[(u + 1) & 1], entry (i, k) at
 // tri_e(i, k). A matrix of two blocks never touches p[1].
-struct TriStage {
-    double d[2][1024];
-    double p[2][1024];
+// The elements keep T's own type (FP32 factors are widened when they are used).
+template <typename E>
+struct TriStageOf {
+    E d[2][1024];
+    E p[2][1024];
 };
+using TriStage = TriStageOf<double>;
 // Swizzled so that A fragments, rows and columns of a block are read and written over all banks.
 __device__ __forceinline__ int tri_e(int i, int k) { return i * 32 + (k ^ (((i & 3) << 2) | ((i >> 2) & 3))); }
 
-// A[0] of the global matrix to shared memory, asynchronously; zero when !valid (nothing is read).
-__device__ __forceinline__ void tri_copy(double* dst, const double* src, bool valid) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"((unsigned)__cvta_generic_to_shared(dst)),
-                 "l"(src), "r"(valid ? 8 : 0)
+// One element to shared memory, asynchronously; zero when !valid (nothing is read).
+template <typename E>
+__device__ __forceinline__ void tri_copy(E* dst, const E* src, bool valid) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;" ::"r"((unsigned)__cvta_generic_to_shared(dst)),
+                 "l"(src), "n"((int)sizeof(E)), "r"(valid ? (int)sizeof(E) : 0)
                  : "memory");
 }
 
@@ -63,8 +67,8 @@ __device__ __forceinline__ void tri_dmma(double& d0, double& d1, double a, doubl
 // One sweep of a team of NW >= 2 warps (team.sync() is its barrier). T(i, k) = A[i * rs + k * cs];
 // lower and ascending, or upper and descending (DESC). X holds ceil(n / 32) * 32 rows. On entry
 // every warp must see X; on return every warp does.
-template <TriDiag MODE, bool DESC, typename Team>
-__device__ __forceinline__ void tri_sweep(const double* A, size_t rs, size_t cs, int n, double* X, TriStage& buf,
+template <TriDiag MODE, bool DESC, typename E, typename Team>
+__device__ __forceinline__ void tri_sweep(const E* A, size_t rs, size_t cs, int n, double* X, TriStageOf<E>& buf,
                                           int NW, const Team& team) {
     const int tid = team.tid(), lane = tid & 31, warp = tid >> 5;
     const int q = lane & 3, r8 = lane >> 2;
@@ -75,20 +79,20 @@ __device__ __forceinline__ void tri_sweep(const double* A, size_t rs, size_t cs,
 
     // Warps first, first + count, .. : a share of the copies for the u-th block in sweep order.
     auto stage = [&](int u, int share, int shares) {
-        double *bd = buf.d[u & 1], *bp = buf.p[(u + 1) & 1];
+        E *bd = buf.d[u & 1], *bp = buf.p[(u + 1) & 1];
         const int j0 = block_of(u) * 32, p0 = u > 0 ? block_of(u - 1) * 32 : 0;
         for (int e = share; e < 32; e += shares) {
             const int i = rs == 1 ? lane : e, k = rs == 1 ? e : lane;   // lanes along the contiguous direction
             const bool vi = j0 + i < n;
             const bool vd = vi && j0 + k < n, vp = vi && p0 + k < n;
-            const double* row = A + (j0 + i) * rs;
+            const E* row = A + (j0 + i) * rs;
             tri_copy(&bd[tri_e(i, k)], vd ? row + (j0 + k) * cs : A, vd);
             if (u > 0) tri_copy(&bp[tri_e(i, k)], vp ? row + (p0 + k) * cs : A, vp);
         }
     };
     // Warp 0: applies the predecessor's solution to the rows of the u-th block and solves them.
     auto lead = [&](int u) {
-        const double *bd = buf.d[u & 1], *bp = buf.p[(u + 1) & 1];
+        const E *bd = buf.d[u & 1], *bp = buf.p[(u + 1) & 1];
         const int j0 = block_of(u) * 32;
         if (u > 0) {
             const int p0 = block_of(u - 1) * 32;
@@ -103,7 +107,7 @@ __device__ __forceinline__ void tri_sweep(const double* A, size_t rs, size_t cs,
             for (int s = 0; s < 8; ++s) {
                 const double b = -X[tri_x(p0 + kof(s), r8)];
 #pragma unroll
-                for (int t = 0; t < 4; ++t) tri_dmma(c[t][0], c[t][1], bp[tri_e(8 * t + r8, kof(s))], b);
+                for (int t = 0; t < 4; ++t) tri_dmma(c[t][0], c[t][1], (double)bp[tri_e(8 * t + r8, kof(s))], b);
             }
 #pragma unroll
             for (int t = 0; t < 4; ++t)
@@ -117,11 +121,11 @@ __device__ __forceinline__ void tri_sweep(const double* A, size_t rs, size_t cs,
             double2 c = *xi;
             double l[8];
 #pragma unroll
-            for (int k = 0; k < 8; ++k) l[k] = bd[tri_e(i, 8 * t + k)];
+            for (int k = 0; k < 8; ++k) l[k] = (double)bd[tri_e(i, 8 * t + k)];
             Divisor v;
             bool slow = false;   // a diagonal entry of the piece that div_fast cannot take
             if constexpr (MODE != TriDiag::Unit) {
-                v = make_divisor(j0 + i < n ? bd[tri_e(i, i)] : 1.0);
+                v = make_divisor(j0 + i < n ? (double)bd[tri_e(i, i)] : 1.0);
                 if (MODE == TriDiag::Divide) slow = __any_sync(kFullMask, !div_fast_den(v.d));
             }
 #pragma unroll
@@ -158,7 +162,7 @@ __device__ __forceinline__ void tri_sweep(const double* A, size_t rs, size_t cs,
                 double2 cw = *xw;
 #pragma unroll
                 for (int h = 0; h < 2; ++h)
-                    tri_dmma(cw.x, cw.y, bd[tri_e(iw, 8 * t + (DESC ? 7 - 4 * h - q : 4 * h + q))], b[h]);
+                    tri_dmma(cw.x, cw.y, (double)bd[tri_e(iw, 8 * t + (DESC ? 7 - 4 * h - q : 4 * h + q))], b[h]);
                 *xw = cw;
             }
             __syncwarp();
@@ -181,7 +185,8 @@ __device__ __forceinline__ void tri_sweep(const double* A, size_t rs, size_t cs,
             const int lo = DESC ? 0 : (jn + 1) * 32, hi = DESC ? jn * 32 : n;
             const int pairs = (hi - lo + 15) / 16;
             if (warp - 1 < pairs) {
-                double b[8], a0[8], a1[8];
+                double b[8];
+                E a0[8], a1[8];
 #pragma unroll
                 for (int s8 = 0; s8 < 8; ++s8) b[s8] = -X[tri_x(b0 + kof(s8), r8)];
                 auto load = [&](int p) {
@@ -189,8 +194,8 @@ __device__ __forceinline__ void tri_sweep(const double* A, size_t rs, size_t cs,
 #pragma unroll
                     for (int s8 = 0; s8 < 8; ++s8) {
                         const int k = b0 + kof(s8);
-                        a0[s8] = (i0 < hi && k < n) ? A[i0 * rs + k * cs] : 0.0;
-                        a1[s8] = (i1 < hi && k < n) ? A[i1 * rs + k * cs] : 0.0;
+                        a0[s8] = (i0 < hi && k < n) ? A[i0 * rs + k * cs] : E(0);
+                        a1[s8] = (i1 < hi && k < n) ? A[i1 * rs + k * cs] : E(0);
                     }
                 };
                 load(warp - 1);
@@ -198,7 +203,7 @@ __device__ __forceinline__ void tri_sweep(const double* A, size_t rs, size_t cs,
                     const int i0 = lo + 16 * p + r8, i1 = i0 + 8;
                     double u0[8], u1[8];
 #pragma unroll
-                    for (int s8 = 0; s8 < 8; ++s8) { u0[s8] = a0[s8]; u1[s8] = a1[s8]; }
+                    for (int s8 = 0; s8 < 8; ++s8) { u0[s8] = (double)a0[s8]; u1[s8] = (double)a1[s8]; }
                     if (p + NW - 1 < pairs) load(p + NW - 1);
                     double2 c0 = *reinterpret_cast<const double2*>(&X[tri_x(i0, 2 * q)]);
                     double2 c1 = *reinterpret_cast<const double2*>(&X[tri_x(i1, 2 * q)]);
