@@ -112,10 +112,7 @@ struct CholRefineSmem {
     double X[NMAX * kTriRhs];      // solution
     double W[NMAX * kTriRhs];      // residual, then correction
     double red[2][16][kTriRhs];
-    TriStageOf<float> st;          // orders up to 32 use st.d[0] alone
-    static constexpr size_t bytes() {
-        return sizeof(CholRefineSmem) - (NMAX <= 32 ? 3 * sizeof(float) * 1024 : 0);
-    }
+    TriStageOf<float> st;
 };
 
 // W -= A X, A symmetric with its lower triangle stored; W and X hold npad >= n rows (zero past n).
@@ -254,6 +251,235 @@ dsposv_refine_vkernel(WorkList wl, const int* n_arr, const int* nrhs_arr, double
     }
 }
 
+// ---- refinement of the small orders: one block per instance, thread t = row t, NT >= n, R right-hand
+// sides at a time in FP32 corrections. Up to 32 rows the tensor-core form's block barriers and eight
+// columns cost more than they save (10,000 x 32^2, 8 RHS: 504 against 585 us), up to 64 with at most
+// four right-hand sides too (2,000 to 10,000 small orders, few RHS: 0.47 against 0.62 ms). ----
+template <int NT, int R>
+struct CholRowRefineSmem {
+    static constexpr int NBLK = NT / 32;
+    float  inv[NBLK][32][33];      // L_JJ^-1 of each 32x32 diagonal block
+    float  sx[2][32][R];           // solved values of the current block (double-buffered)
+    float  sb[NBLK][32][R];        // per-warp staging of a block's right-hand sides
+    double xs[NT][R];              // FP64 solution, shared for the residual
+    double red[2][NBLK][R];
+};
+
+// L_JJ^-1 (lower, non-unit) of diagonal block J of SA, by warp J: lane j forms column j.
+template <int NT, int R>
+__device__ __forceinline__ void chol_invert_diag_block(const float* __restrict__ SA, int n, int J, int lane,
+                                                       CholRowRefineSmem<NT, R>& sh) {
+    const int j0 = J * 32;
+    float (&T)[32][33] = sh.inv[J];
+#pragma unroll 4
+    for (int k = 0; k < 32; ++k)
+        T[lane][k] = (j0 + lane < n && j0 + k < n) ? (k <= lane ? SA[j0 + lane + (size_t)(j0 + k) * n] : 0.0f)
+                                                   : (lane == k ? 1.0f : 0.0f);
+    __syncwarp();
+    float x[32];
+    static_for<0, 32>([&](auto ic) {
+        constexpr int i = decltype(ic)::value;
+        float s = (i == lane) ? 1.0f : 0.0f;
+#pragma unroll
+        for (int k = 0; k < i; ++k) s = fmaf(-T[i][k], x[k], s);
+        x[i] = (i < lane) ? 0.0f : s / T[i][i];
+    });
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < 32; ++i) T[i][lane] = x[i];
+    __syncwarp();
+}
+
+// L L^T c = b in single precision for the R right-hand sides in f (thread t = row t).
+template <int NT, int R>
+__device__ __forceinline__ void chol_refine_solve(const float* __restrict__ SA, int n, float (&f)[R],
+                                                  CholRowRefineSmem<NT, R>& sh) {
+    const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+    const int nblk = (n + 31) / 32;
+    auto diag_step = [&](int J, bool transposed, int buf) {
+#pragma unroll
+        for (int r = 0; r < R; ++r) sh.sb[w][lane][r] = f[r];
+        __syncwarp();
+        float x[R];
+#pragma unroll
+        for (int r = 0; r < R; ++r) x[r] = 0.0f;
+#pragma unroll 8
+        for (int k = 0; k < 32; ++k) {
+            const float l = transposed ? sh.inv[J][k][lane] : sh.inv[J][lane][k];
+#pragma unroll
+            for (int r = 0; r < R; ++r) x[r] = fmaf(l, sh.sb[w][k][r], x[r]);
+        }
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            f[r] = x[r];
+            sh.sx[buf][lane][r] = x[r];
+        }
+    };
+    // forward: L y = b, blocks ascending; rows below take L(i, block) * y_block
+    for (int J = 0; J < nblk; ++J) {
+        const int j0 = J * 32, buf = J & 1;
+        float lv[32];
+        const bool below = (w > J && t < n);
+        if (below) {
+#pragma unroll
+            for (int k = 0; k < 32; ++k) lv[k] = (j0 + k < n) ? SA[t + (size_t)(j0 + k) * n] : 0.0f;
+        }
+        if (w == J) diag_step(J, false, buf);
+        __syncthreads();
+        if (below) {
+#pragma unroll
+            for (int k = 0; k < 32; ++k) {
+#pragma unroll
+                for (int r = 0; r < R; ++r) f[r] = fmaf(-lv[k], sh.sx[buf][k][r], f[r]);
+            }
+        }
+    }
+    // backward: L^T x = y, blocks descending; rows above take L(block, i)^T * x_block
+    for (int J = nblk - 1; J >= 0; --J) {
+        const int j0 = J * 32, buf = (2 * nblk - 1 - J) & 1;
+        float uv[32];
+        const bool above = (w < J);
+        if (above) {
+#pragma unroll
+            for (int k = 0; k < 32; ++k) uv[k] = (j0 + k < n) ? SA[j0 + k + (size_t)t * n] : 0.0f;
+        }
+        if (w == J) diag_step(J, true, buf);
+        __syncthreads();
+        if (above) {
+#pragma unroll
+            for (int k = 0; k < 32; ++k) {
+#pragma unroll
+                for (int r = 0; r < R; ++r) f[r] = fmaf(-uv[k], sh.sx[buf][k][r], f[r]);
+            }
+        }
+    }
+}
+
+template <int NT, int R>
+__global__ void __launch_bounds__(NT, (NT >= 512 ? 1 : 512 / NT))
+dsposv_refine_rows_vkernel(WorkList wl, const int* n_arr, const int* nrhs_arr, double** dA_array, const int* ldda,
+                      double** dB_array, const int* lddb, double** dX_array, const int* lddx, float** dS_array,
+                      CholMixedWs ws, int* iter_array) {
+    extern __shared__ __align__(16) unsigned char chol_refine_smem[];
+    CholRowRefineSmem<NT, R>& sh = *reinterpret_cast<CholRowRefineSmem<NT, R>*>(chol_refine_smem);
+    const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+    for (int it = blockIdx.x; it < wl.size(); it += gridDim.x) {
+        const int id = wl.at(it);
+        if (iter_array[id] < 0) continue;        // conversion already failed (block-uniform)
+        const int n = n_arr[id], nrhs = nrhs_arr[id];
+        if (ws.sinfo[id] != 0) {                 // not positive definite in single precision
+            if (t == 0) { iter_array[id] = -3; ws.fkey[id] = n; }
+            continue;
+        }
+        const double* A = dA_array[id];
+        const double* B = dB_array[id];
+        double* X = dX_array[id];
+        const int lda = ldda[id], ldb = lddb[id], ldx = lddx[id];
+        const float* SA = dS_array[id];
+        const double cte = ws.anrm[id] * (DBL_EPSILON * 0.5) * sqrt((double)n);
+        const int nblk = (n + 31) / 32;
+        for (int J = w; J < nblk; J += NT / 32) chol_invert_diag_block<NT, R>(SA, n, J, lane, sh);
+        __syncthreads();
+        int iter_out = 0;
+        for (int c0 = 0; c0 < nrhs && iter_out >= 0; c0 += R) {
+            double b[R], x[R], res[R];
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+                b[r] = (t < n && c0 + r < nrhs) ? B[t + (size_t)(c0 + r) * ldb] : 0.0;
+                x[r] = 0.0;
+                res[r] = b[r];
+            }
+            int iiter = 0, stalls = 0;
+            double prev_ratio = 1e300;
+            for (;;) {
+                bool ovf = false;
+                float f[R];
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                    ovf |= !(fabs(res[r]) <= (double)FLT_MAX);
+                    f[r] = (float)res[r];
+                }
+                if (__syncthreads_or(ovf)) { iter_out = -2; break; }
+                chol_refine_solve<NT, R>(SA, n, f, sh);
+                if (t < n) {
+#pragma unroll
+                    for (int r = 0; r < R; ++r) {
+                        x[r] += (double)f[r];
+                        sh.xs[t][r] = x[r];
+                    }
+                }
+                __syncthreads();
+                // R = B - A X with A symmetric, lower triangle stored
+#pragma unroll
+                for (int r = 0; r < R; ++r) res[r] = b[r];
+                if (t < n) {
+#pragma unroll 8
+                    for (int j = 0; j <= t; ++j) {
+                        const double a = A[t + (size_t)j * lda];
+#pragma unroll
+                        for (int r = 0; r < R; ++r) res[r] = fma(-a, sh.xs[j][r], res[r]);
+                    }
+#pragma unroll 8
+                    for (int j = t + 1; j < n; ++j) {
+                        const double a = A[j + (size_t)t * lda];
+#pragma unroll
+                        for (int r = 0; r < R; ++r) res[r] = fma(-a, sh.xs[j][r], res[r]);
+                    }
+                }
+                double xn[R], rn[R];
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                    xn[r] = (t < n && c0 + r < nrhs) ? fabs(x[r]) : 0.0;
+                    rn[r] = (t < n && c0 + r < nrhs) ? fabs(res[r]) : 0.0;
+                }
+                // block-wide maxima per right-hand side
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                    for (int off = 16; off > 0; off >>= 1) {
+                        xn[r] = fmax(xn[r], __shfl_xor_sync(kFullMask, xn[r], off));
+                        rn[r] = fmax(rn[r], __shfl_xor_sync(kFullMask, rn[r], off));
+                    }
+                }
+                __syncthreads();
+                if (lane == 0) {
+#pragma unroll
+                    for (int r = 0; r < R; ++r) { sh.red[0][w][r] = xn[r]; sh.red[1][w][r] = rn[r]; }
+                }
+                __syncthreads();
+                bool ok = true;
+                double ratio = 0.0;
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                    double xm = 0.0, rm = 0.0;
+                    for (int k = 0; k < NT / 32; ++k) { xm = fmax(xm, sh.red[0][k][r]); rm = fmax(rm, sh.red[1][k][r]); }
+                    if (c0 + r < nrhs) {
+                        ok &= (rm <= xm * cte);
+                        ratio = fmax(ratio, rm / fmax(xm * cte, DBL_MIN));
+                    }
+                }
+                if (ok) break;
+                ++iiter;
+                stalls = (ratio > 0.5 * prev_ratio) ? stalls + 1 : 0;
+                prev_ratio = ratio;
+                if (iiter >= kCholItermax || stalls >= 2) { iter_out = -kCholItermax - 1; break; }
+            }
+            if (iter_out < 0) break;
+            iter_out = max(iter_out, iiter);
+            if (t < n) {
+#pragma unroll
+                for (int r = 0; r < R; ++r)
+                    if (c0 + r < nrhs) X[t + (size_t)(c0 + r) * ldx] = x[r];
+            }
+            __syncthreads();
+        }
+        if (t == 0) {
+            iter_array[id] = iter_out;
+            ws.fkey[id] = iter_out < 0 ? n : 0;
+        }
+        __syncthreads();
+    }
+}
+
 // ---- 3. fallback helper: X = B for the listed instances ----
 __global__ void copy_rhs_vkernel(WorkList wl, const int* n_arr, const int* nrhs_arr, double** dB_array,
                                  const int* lddb, double** dX_array, const int* lddx) {
@@ -301,29 +527,40 @@ static int persistent_grid(K kernel, int threads, size_t smem, int bound) {
 }
 
 template <int NT>
-static void launch_bucket_stage(int stage, const WorkList& wl, int batch, const int* n, const int* nrhs, double** A,
+static void launch_bucket_stage(int stage, const WorkList& wl, int batch, int max_nrhs, const int* n,
+                                const int* nrhs, double** A,
                                 const int* lda, double** B, const int* ldb, double** X, const int* ldx, float** S,
                                 const CholMixedWs& ws, int* iter, cudaStream_t s) {
     if (stage == 0) {
         auto k = dlat2s_norm_vkernel<NT>;
         k<<<persistent_grid(k, NT, 0, batch), NT, 0, s>>>(wl, n, A, lda, S, ws, iter);
+    } else if (NT == 32 || (NT == 64 && max_nrhs <= 4)) {
+        if constexpr (NT <= 64) {
+            constexpr int R = 4;
+            auto k = dsposv_refine_rows_vkernel<NT, R>;
+            const int smem = (int)sizeof(CholRowRefineSmem<NT, R>);
+            ensure_dynamic_smem((const void*)k, smem);
+            k<<<persistent_grid(k, NT, smem, batch), NT, smem, s>>>(wl, n, nrhs, A, lda, B, ldb, X, ldx, S, ws, iter);
+        }
     } else {
-        constexpr int RT = NT <= 128 ? 64 : NT / 2;   // refinement threads: two warps up to n = 128
-        auto k = dsposv_refine_vkernel<NT, RT>;
-        const int smem = (int)CholRefineSmem<NT>::bytes();
-        ensure_dynamic_smem((const void*)k, smem);
-        k<<<persistent_grid(k, RT, smem, batch), RT, smem, s>>>(wl, n, nrhs, A, lda, B, ldb, X, ldx, S, ws, iter);
+        if constexpr (NT > 32) {
+            constexpr int RT = NT <= 128 ? 64 : NT / 2;   // refinement threads: two warps up to n = 128
+            auto k = dsposv_refine_vkernel<NT, RT>;
+            const int smem = (int)sizeof(CholRefineSmem<NT>);
+            ensure_dynamic_smem((const void*)k, smem);
+            k<<<persistent_grid(k, RT, smem, batch), RT, smem, s>>>(wl, n, nrhs, A, lda, B, ldb, X, ldx, S, ws, iter);
+        }
     }
 }
 
-static void bucket_stage(int edge, int stage, const WorkList& wl, int batch, const int* n, const int* nrhs,
+static void bucket_stage(int edge, int stage, const WorkList& wl, int batch, int max_nrhs, const int* n, const int* nrhs,
                          double** A, const int* lda, double** B, const int* ldb, double** X, const int* ldx,
                          float** S, const CholMixedWs& ws, int* iter, cudaStream_t s) {
-    if (edge <= 32) launch_bucket_stage<32>(stage, wl, batch, n, nrhs, A, lda, B, ldb, X, ldx, S, ws, iter, s);
-    else if (edge <= 64) launch_bucket_stage<64>(stage, wl, batch, n, nrhs, A, lda, B, ldb, X, ldx, S, ws, iter, s);
-    else if (edge <= 128) launch_bucket_stage<128>(stage, wl, batch, n, nrhs, A, lda, B, ldb, X, ldx, S, ws, iter, s);
-    else if (edge <= 256) launch_bucket_stage<256>(stage, wl, batch, n, nrhs, A, lda, B, ldb, X, ldx, S, ws, iter, s);
-    else launch_bucket_stage<512>(stage, wl, batch, n, nrhs, A, lda, B, ldb, X, ldx, S, ws, iter, s);
+    if (edge <= 32) launch_bucket_stage<32>(stage, wl, batch, max_nrhs, n, nrhs, A, lda, B, ldb, X, ldx, S, ws, iter, s);
+    else if (edge <= 64) launch_bucket_stage<64>(stage, wl, batch, max_nrhs, n, nrhs, A, lda, B, ldb, X, ldx, S, ws, iter, s);
+    else if (edge <= 128) launch_bucket_stage<128>(stage, wl, batch, max_nrhs, n, nrhs, A, lda, B, ldb, X, ldx, S, ws, iter, s);
+    else if (edge <= 256) launch_bucket_stage<256>(stage, wl, batch, max_nrhs, n, nrhs, A, lda, B, ldb, X, ldx, S, ws, iter, s);
+    else launch_bucket_stage<512>(stage, wl, batch, max_nrhs, n, nrhs, A, lda, B, ldb, X, ldx, S, ws, iter, s);
 }
 
 bool dsposv_vbatched_supported(int max_n) { return max_n <= 512; }
@@ -358,9 +595,9 @@ magma_int_t dsposv_var(const int* n, const int* nrhs, double** A, const int* lda
     for (int b = top; b >= 0; --b) {
         cudaStream_t sb = queue_aux(queue, top - b);
         const WorkList wl{lists + (size_t)b * batch, counts + b, 0};
-        bucket_stage(kCholEdges[b], 0, wl, batch, n, nrhs, A, lda, B, ldb, X, ldx, S, ws, iter, sb);
+        bucket_stage(kCholEdges[b], 0, wl, batch, max_nrhs, n, nrhs, A, lda, B, ldb, X, ldx, S, ws, iter, sb);
         chol_bucket<float>(b, wl, batch, true, sz32, false, S, nullptr, ws.sinfo, true, false, 0, sb);
-        bucket_stage(kCholEdges[b], 1, wl, batch, n, nrhs, A, lda, B, ldb, X, ldx, S, ws, iter, sb);
+        bucket_stage(kCholEdges[b], 1, wl, batch, max_nrhs, n, nrhs, A, lda, B, ldb, X, ldx, S, ws, iter, sb);
     }
     queue_join(queue);
     if ((rc = launch_status())) return rc;
