@@ -416,6 +416,28 @@ __device__ __forceinline__ int tc_kmajor(int row, int k) {   // float index of (
     return (((row >> 3) * 8 + (k >> 2)) * 8 + (row & 7)) * 4 + (k & 3);
 }
 
+// The first `left` of 32 consecutive values (zero past them), four a load where `vec` says that the
+// address allows it: a thread's row of an operand stored along k is one cache line, and one load
+// per value made each of a warp's loads touch 32 lines.
+__device__ __forceinline__ void tc_load_k(float (&x)[kTcGemmKc], const float* p, int left, bool vec) {
+#pragma unroll
+    for (int q = 0; q < kTcGemmKc; q += 4) {
+        float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (vec && q + 4 <= left) {
+            v = *reinterpret_cast<const float4*>(p + q);
+        } else {
+            if (q < left) v.x = p[q];
+            if (q + 1 < left) v.y = p[q + 1];
+            if (q + 2 < left) v.z = p[q + 2];
+            if (q + 3 < left) v.w = p[q + 3];
+        }
+        x[q] = v.x;
+        x[q + 1] = v.y;
+        x[q + 2] = v.z;
+        x[q + 3] = v.w;
+    }
+}
+
 template <bool TA, bool TB>
 __global__ void __launch_bounds__(128, 3)
 gemm_tc_kernel(GemmSizes g, float alpha, const float* const* __restrict__ A_arr,
@@ -443,6 +465,14 @@ gemm_tc_kernel(GemmSizes g, float alpha, const float* const* __restrict__ A_arr,
     const int tid = threadIdx.x, warp = tid >> 5;
     const int mrows = min(BM, m - i0), ncols = min(BN, n - j0);
     const int npad = (ncols + 15) & ~15;
+    const bool va = ((reinterpret_cast<size_t>(A) | (size_t)lda * 4) & 15) == 0;
+    const bool vb = ((reinterpret_cast<size_t>(B) | (size_t)ldb * 4) & 15) == 0;
+    // C is read after the last product: its lines start towards L2 now
+    if (beta != 0.0f)
+        for (int e = tid; e < 4 * ncols; e += 128) {
+            const int r = 32 * (e & 3), c = e >> 2;
+            if (r < mrows) asm volatile("prefetch.global.L2 [%0];" ::"l"(C + (i0 + r) + (size_t)(j0 + c) * ldc));
+        }
     const uint32_t mbar = tc::smem_addr(&mbar_word);
     if (warp == 0) {
         tc::tmem_alloc(tc::smem_addr(&tmem_base), BN);
@@ -468,9 +498,11 @@ gemm_tc_kernel(GemmSizes g, float alpha, const float* const* __restrict__ A_arr,
 #pragma unroll
         for (int q = 0; q < KC; ++q) {
             const int gk = k0 + q;
-            xa[q] = (tid < mrows && gk < k) ? (TA ? A[gk + (size_t)gi * lda] : A[gi + (size_t)gk * lda]) : 0.0f;
-            xb[q] = (tid < ncols && gk < k) ? (TB ? B[gj + (size_t)gk * ldb] : B[gk + (size_t)gj * ldb]) : 0.0f;
+            if (!TA) xa[q] = (tid < mrows && gk < k) ? A[gi + (size_t)gk * lda] : 0.0f;
+            if (TB) xb[q] = (tid < ncols && gk < k) ? B[gj + (size_t)gk * ldb] : 0.0f;
         }
+        if (TA) tc_load_k(xa, A + k0 + (size_t)gi * lda, tid < mrows ? k - k0 : 0, va);
+        if (!TB) tc_load_k(xb, B + k0 + (size_t)gj * ldb, tid < ncols ? k - k0 : 0, vb);
         if (tid < mrows) {
 #pragma unroll
             for (int q = 0; q < KC; q += 4) {
