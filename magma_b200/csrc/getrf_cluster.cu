@@ -15,6 +15,10 @@ getrf_cluster_kernel(WorkList wl, LuSizes sz, double** dA_array, int** ipiv_arra
     extern __shared__ __align__(16) unsigned char getrf_cluster_smem[];
     auto& sh = *reinterpret_cast<ClusterLuShared<NB, NT, CS>*>(getrf_cluster_smem);
     const int rank = CS == 1 ? 0 : (int)cooperative_groups::this_cluster().block_rank();
+    // A block's first pivot candidate goes to its peers before anything of the panel makes the
+    // cluster meet, and a peer's shared memory may be stored to only once that peer runs. The
+    // barrier that ends each matrix does the same for the matrices after it, and for the exit.
+    if constexpr (CS > 1) cluster_sync<CS>();
     for (int w = blockIdx.x / CS; w < wl.size(); w += gridDim.x / CS) {
         const int id = wl.at(w);
         const int m = sz.get_m(id), n = sz.get_n(id), lda = sz.get_lda(id);

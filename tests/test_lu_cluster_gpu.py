@@ -55,3 +55,21 @@ def test_getrf_nopiv_cluster_bit_identical(cuda, m):
     info = mb.dgetrf_nopiv_batched(D)
     assert np.array_equal(info.cpu().numpy(), oinf)
     assert np.array_equal(D.cpu().numpy(), O)
+
+
+@pytest.mark.parametrize("m,n", [(257, 1), (400, 2), (513, 1), (1024, 3)])
+def test_short_factorisations(cuda, m, n):
+    """A panel of one to three steps in more clusters than the machine holds at once: each cluster's
+    first exchange comes right after it starts, while its blocks replace other clusters'."""
+    import torch
+
+    import magma_b200 as mb
+    import oracle
+    A = np.random.default_rng(m).uniform(-1, 1, (1500, n, m))
+    O = A.copy()
+    oip, oinf = oracle.dgetrf_batched(O, m)
+    D = torch.from_numpy(A).to(cuda)
+    ipiv, info = mb.dgetrf_batched(D, m=m)
+    assert np.array_equal(ipiv.cpu().numpy()[:, :n], oip[:, :n])
+    assert np.array_equal(info.cpu().numpy(), oinf)
+    assert np.array_equal(D.cpu().numpy(), O)
