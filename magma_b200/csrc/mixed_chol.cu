@@ -102,9 +102,10 @@ dlat2s_norm_vkernel(WorkList wl, const int* n_arr, double** dA_array, const int*
     }
 }
 
-// ---- 2. refinement: one block of NT threads per instance, n <= NMAX, eight right-hand sides at a
-// time. The correction solves L L^T c = r with the FP32 factor on the FP64 tensor cores
-// (tri_solve.cuh), the residual B - A X is a tensor-core product over the stored triangle (a warp
+// ---- 2. refinement of orders above kCholRowsMax: one block of NT threads per instance, n <= NMAX,
+// eight right-hand sides at a time. The correction solves L L^T c = r with the FP32 factor, widened,
+// in FP64 arithmetic on the tensor cores (tri_solve.cuh); the iteration counts are those of FP32
+// corrections (orders 129..512, 1 to 8 RHS, up to 1,000 instances: all equal). The residual B - A X is a tensor-core product over the stored triangle (a warp
 // per 16 rows). Both read A and L along their contiguous direction whichever triangle an element
 // lies in; the former thread-per-row loops read half of each with 32 lines a load.
 template <int NMAX>
@@ -154,7 +155,7 @@ __device__ __forceinline__ void chol_residual(const double* __restrict__ A, int 
 }
 
 template <int NMAX, int NT>
-__global__ void __launch_bounds__(NT, (NT == 64 ? 8 : NT == 128 ? 4 : 2))
+__global__ void __launch_bounds__(NT, (NT == 128 ? 4 : 2))
 dsposv_refine_vkernel(WorkList wl, const int* n_arr, const int* nrhs_arr, double** dA_array, const int* ldda,
                       double** dB_array, const int* lddb, double** dX_array, const int* lddx, float** dS_array,
                       CholMixedWs ws, int* iter_array) {
@@ -251,10 +252,16 @@ dsposv_refine_vkernel(WorkList wl, const int* n_arr, const int* nrhs_arr, double
     }
 }
 
-// ---- refinement of the small orders: one block per instance, thread t = row t, NT >= n, R right-hand
-// sides at a time in FP32 corrections. Up to 32 rows the tensor-core form's block barriers and eight
-// columns cost more than they save (10,000 x 32^2, 8 RHS: 504 against 585 us), up to 64 with at most
-// four right-hand sides too (2,000 to 10,000 small orders, few RHS: 0.47 against 0.62 ms). ----
+// ---- refinement of orders up to kCholRowsMax: one block per instance, thread t = row t, NT >= n, R
+// right-hand sides at a time in FP32 corrections. The tensor-core form's block barriers and its eight
+// columns cost these orders more than they save (whole call, this form against the other: 10,000
+// x 32^2, 8 RHS 504 against 585 us; orders 33..40, 8 RHS 1,116 against 1,360; 65..128, 1 RHS 2,521
+// against 3,859 and 8 RHS 3,182 against 4,053; 50 orders 65..128, 1 RHS 166 against 244; but 1,000
+// orders 129..256, 1 RHS 1,561 against 1,290). The form follows from the order alone: an instance's
+// solution and iteration count depend neither on what else is in its batch nor on the caller's
+// maximum. ----
+constexpr int kCholRowsMax = 128;
+
 template <int NT, int R>
 struct CholRowRefineSmem {
     static constexpr int NBLK = NT / 32;
@@ -527,40 +534,35 @@ static int persistent_grid(K kernel, int threads, size_t smem, int bound) {
 }
 
 template <int NT>
-static void launch_bucket_stage(int stage, const WorkList& wl, int batch, int max_nrhs, const int* n,
-                                const int* nrhs, double** A,
+static void launch_bucket_stage(int stage, const WorkList& wl, int batch, const int* n, const int* nrhs, double** A,
                                 const int* lda, double** B, const int* ldb, double** X, const int* ldx, float** S,
                                 const CholMixedWs& ws, int* iter, cudaStream_t s) {
     if (stage == 0) {
         auto k = dlat2s_norm_vkernel<NT>;
         k<<<persistent_grid(k, NT, 0, batch), NT, 0, s>>>(wl, n, A, lda, S, ws, iter);
-    } else if (NT == 32 || (NT == 64 && max_nrhs <= 4)) {
-        if constexpr (NT <= 64) {
-            constexpr int R = 4;
-            auto k = dsposv_refine_rows_vkernel<NT, R>;
-            const int smem = (int)sizeof(CholRowRefineSmem<NT, R>);
-            ensure_dynamic_smem((const void*)k, smem);
-            k<<<persistent_grid(k, NT, smem, batch), NT, smem, s>>>(wl, n, nrhs, A, lda, B, ldb, X, ldx, S, ws, iter);
-        }
+    } else if constexpr (NT <= kCholRowsMax) {
+        constexpr int R = 4;
+        auto k = dsposv_refine_rows_vkernel<NT, R>;
+        const int smem = (int)sizeof(CholRowRefineSmem<NT, R>);
+        ensure_dynamic_smem((const void*)k, smem);
+        k<<<persistent_grid(k, NT, smem, batch), NT, smem, s>>>(wl, n, nrhs, A, lda, B, ldb, X, ldx, S, ws, iter);
     } else {
-        if constexpr (NT > 32) {
-            constexpr int RT = NT <= 128 ? 64 : NT / 2;   // refinement threads: two warps up to n = 128
-            auto k = dsposv_refine_vkernel<NT, RT>;
-            const int smem = (int)sizeof(CholRefineSmem<NT>);
-            ensure_dynamic_smem((const void*)k, smem);
-            k<<<persistent_grid(k, RT, smem, batch), RT, smem, s>>>(wl, n, nrhs, A, lda, B, ldb, X, ldx, S, ws, iter);
-        }
+        constexpr int RT = NT / 2;   // refinement threads
+        auto k = dsposv_refine_vkernel<NT, RT>;
+        const int smem = (int)sizeof(CholRefineSmem<NT>);
+        ensure_dynamic_smem((const void*)k, smem);
+        k<<<persistent_grid(k, RT, smem, batch), RT, smem, s>>>(wl, n, nrhs, A, lda, B, ldb, X, ldx, S, ws, iter);
     }
 }
 
-static void bucket_stage(int edge, int stage, const WorkList& wl, int batch, int max_nrhs, const int* n, const int* nrhs,
+static void bucket_stage(int edge, int stage, const WorkList& wl, int batch, const int* n, const int* nrhs,
                          double** A, const int* lda, double** B, const int* ldb, double** X, const int* ldx,
                          float** S, const CholMixedWs& ws, int* iter, cudaStream_t s) {
-    if (edge <= 32) launch_bucket_stage<32>(stage, wl, batch, max_nrhs, n, nrhs, A, lda, B, ldb, X, ldx, S, ws, iter, s);
-    else if (edge <= 64) launch_bucket_stage<64>(stage, wl, batch, max_nrhs, n, nrhs, A, lda, B, ldb, X, ldx, S, ws, iter, s);
-    else if (edge <= 128) launch_bucket_stage<128>(stage, wl, batch, max_nrhs, n, nrhs, A, lda, B, ldb, X, ldx, S, ws, iter, s);
-    else if (edge <= 256) launch_bucket_stage<256>(stage, wl, batch, max_nrhs, n, nrhs, A, lda, B, ldb, X, ldx, S, ws, iter, s);
-    else launch_bucket_stage<512>(stage, wl, batch, max_nrhs, n, nrhs, A, lda, B, ldb, X, ldx, S, ws, iter, s);
+    if (edge <= 32) launch_bucket_stage<32>(stage, wl, batch, n, nrhs, A, lda, B, ldb, X, ldx, S, ws, iter, s);
+    else if (edge <= 64) launch_bucket_stage<64>(stage, wl, batch, n, nrhs, A, lda, B, ldb, X, ldx, S, ws, iter, s);
+    else if (edge <= 128) launch_bucket_stage<128>(stage, wl, batch, n, nrhs, A, lda, B, ldb, X, ldx, S, ws, iter, s);
+    else if (edge <= 256) launch_bucket_stage<256>(stage, wl, batch, n, nrhs, A, lda, B, ldb, X, ldx, S, ws, iter, s);
+    else launch_bucket_stage<512>(stage, wl, batch, n, nrhs, A, lda, B, ldb, X, ldx, S, ws, iter, s);
 }
 
 bool dsposv_vbatched_supported(int max_n) { return max_n <= 512; }
@@ -595,9 +597,9 @@ magma_int_t dsposv_var(const int* n, const int* nrhs, double** A, const int* lda
     for (int b = top; b >= 0; --b) {
         cudaStream_t sb = queue_aux(queue, top - b);
         const WorkList wl{lists + (size_t)b * batch, counts + b, 0};
-        bucket_stage(kCholEdges[b], 0, wl, batch, max_nrhs, n, nrhs, A, lda, B, ldb, X, ldx, S, ws, iter, sb);
+        bucket_stage(kCholEdges[b], 0, wl, batch, n, nrhs, A, lda, B, ldb, X, ldx, S, ws, iter, sb);
         chol_bucket<float>(b, wl, batch, true, sz32, false, S, nullptr, ws.sinfo, true, false, 0, sb);
-        bucket_stage(kCholEdges[b], 1, wl, batch, max_nrhs, n, nrhs, A, lda, B, ldb, X, ldx, S, ws, iter, sb);
+        bucket_stage(kCholEdges[b], 1, wl, batch, n, nrhs, A, lda, B, ldb, X, ldx, S, ws, iter, sb);
     }
     queue_join(queue);
     if ((rc = launch_status())) return rc;

@@ -77,6 +77,29 @@ def test_dsposv_vbatched_fallbacks(cuda):
         assert _bwd(As[i], Xs[i], Bs[i]) <= 1e-14, i
 
 
+def test_dsposv_vbatched_independent_of_the_batch(cuda):
+    """An instance's solution and iteration count follow from the instance alone: not from the
+    caller's maximum of right-hand sides, nor from another instance with more of them."""
+    import magma_b200 as mb
+    from magma_b200.api import VarBatch
+    ns = np.repeat([20, 32, 33, 40, 64, 65, 128, 129, 256], 12)
+    rng = np.random.default_rng(8)
+    nrhs = rng.integers(1, 5, len(ns))
+    As = [np.ascontiguousarray(T.spd_gram(int(n), 44, i)) for i, n in enumerate(ns)]
+    Bs = [rng.standard_normal((int(r), int(n))) for n, r in zip(ns, nrhs)]
+    extra = (np.ascontiguousarray(T.spd_gram(50, 45, 0)), rng.standard_normal((8, 50)))
+    results = []
+    for most, more in ((4, False), (8, False), (8, True)):
+        a, b, n, r = (As + [extra[0]], Bs + [extra[1]], np.append(ns, 50), np.append(nrhs, 8)) if more else (As, Bs, ns, nrhs)
+        X, it, info = mb.dsposv_vbatched(VarBatch(a, cuda), VarBatch(b, cuda), n, r, max_sizes=(256, most))
+        assert not info.cpu().numpy().any()
+        results.append((X.unpack()[:len(ns)], it.cpu().numpy()[:len(ns)]))
+    for X, it in results[1:]:
+        assert np.array_equal(it, results[0][1])
+        for i in range(len(ns)):
+            assert np.array_equal(X[i], results[0][0][i]), (i, ns[i])
+
+
 def test_dsposv_vbatched_argument_errors(cuda):
     import magma_b200 as mb
     from magma_b200.api import VarBatch
