@@ -22,11 +22,11 @@ magma_int_t getrs_small(const WorkList& wl, int bound, bool persistent, bool tra
                         int max_nrhs, T** A, int** ipiv, T** B, cudaStream_t s);
 
 // Blocked LU family (getrf_blocked.cu), m <= 1024: one matrix per thread block, or in FP64
-// getrf per thread-block cluster.
+// getrf per thread-block cluster. No instance has more than max_m rows or max_n columns.
 bool blocked_lu_supported(int max_m);
 template <typename T>
-magma_int_t getrf_blocked(const WorkList& wl, int bound, bool persistent, const LuSizes& sz, int max_m, T** A,
-                          int** ipiv, int* info, cudaStream_t s);
+magma_int_t getrf_blocked(const WorkList& wl, int bound, bool persistent, const LuSizes& sz, int max_m, int max_n,
+                          T** A, int** ipiv, int* info, cudaStream_t s);
 // FP64 LU, one matrix per thread-block cluster (getrf_cluster.cu): m <= 1024.
 magma_int_t getrf_cluster(const WorkList& wl, int bound, bool persistent, const LuSizes& sz, int max_m, double** A,
                           int** ipiv, int* info, cudaStream_t s);

@@ -24,8 +24,9 @@
 // Every element receives its updates as single fma's in increasing step
 // order, exactly like the unblocked dgetf2 (DGER per step), so factors,
 // pivots and info are bit-identical to the oracle restatement at every size.
-// FP32 getrf runs this kernel, and so do the teams of the one-launch variable-size FP64 LU
-// (lu_queue.cuh); other FP64 calls run the cluster kernel (cluster_lu.cuh).
+// FP32 getrf runs this kernel, and so do tall FP64 matrices (getrf_blocked.cu) and the teams of the
+// one-launch variable-size FP64 LU (lu_queue.cuh); other FP64 calls run the cluster kernel
+// (cluster_lu.cuh).
 #pragma once
 
 #include "small_lu.cuh"

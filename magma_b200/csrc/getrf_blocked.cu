@@ -1,6 +1,6 @@
 // getrf_blocked.cu -- kernels and host dispatch of the blocked batched LU
-// (one matrix per thread block, up to 1024 rows): FP32. FP64 runs getrf_cluster.cu
-// and getrs_tc.cu.
+// (one matrix per thread block, up to 1024 rows): FP32, and FP64 where a matrix is tall
+// (getrf_tall). Other FP64 calls run getrf_cluster.cu and getrs_tc.cu.
 #include "internal.h"
 #include "blocked_lu.cuh"
 #include "getrs_blocked.cuh"
@@ -65,10 +65,36 @@ static void launch_getrf_blocked(const WorkList& wl, int bound, bool persistent,
     k<<<blocked_grid(k, NT, bound, persistent, smem), NT, smem, s>>>(wl, sz, A, ipiv, info);
 }
 
+// FP64 matrices of more rows than one block of the cluster kernel holds, but few columns: nearly all
+// of their time is panel steps, which cross the cluster there and cost one block's barrier here.
+// Measured, this kernel against the cluster (us):
+//   257..512 rows (two blocks a matrix): 2,000 x (300 x 32) 341 against 634, (512 x 128) 2,898
+//   against 3,390, (512 x 192) 5,705 against 6,050; 16 x (300 x 96) 124 against 135, (300 x 128)
+//   182 against 182, (300 x 192) 334 against 284;
+//   513..1024 rows (four blocks): 2,000 x (1024 x 8) 191 against 432, (1024 x 96) 4,293 against
+//   5,620, 300 x (1024 x 128) 1,418 against 1,361; 16 x (600 x 16) 26 against 30, (1024 x 32) 60
+//   against 48.
+// The lines lie where the two meet. They move with the matrices per SM: up to half a matrix an SM, a
+// cluster's blocks have SMs to themselves; from there on they share them, and what counts is the work
+// of all. 2,000 x (600 x 128) 5,074 against 6,982, (800 x 160) 9,063 against 9,812; 100 x (600 x 128)
+// 366 against 473.
+static bool getrf_tall(int max_m, int max_n, int bound) {
+    if (max_m <= 256) return false;
+    const float per_sm = (float)bound / device_sm_count();
+    if (max_m <= 512) return max_n <= (per_sm > 4 ? 192 : per_sm > 0.5f ? 160 : 96);
+    if (per_sm > 0.5f && per_sm <= 1) return max_n <= 128;   // one wave of blocks, two of clusters
+    return max_n <= (per_sm > 6 ? 160 : per_sm > 2 ? 128 : per_sm > 1 ? 96 : 16);
+}
+
 template <typename T>
-magma_int_t getrf_blocked(const WorkList& wl, int bound, bool persistent, const LuSizes& sz, int max_m, T** A,
-                          int** ipiv, int* info, cudaStream_t s) {
+magma_int_t getrf_blocked(const WorkList& wl, int bound, bool persistent, const LuSizes& sz, int max_m, int max_n,
+                          T** A, int** ipiv, int* info, cudaStream_t s) {
     if constexpr (std::is_same<T, double>::value) {
+        if (getrf_tall(max_m, max_n, bound)) {
+            if (max_m <= 512) launch_getrf_blocked<T, 32, 512, 128, 8>(wl, bound, persistent, sz, A, ipiv, info, s);
+            else launch_getrf_blocked<T, 16, 1024, 128, 2>(wl, bound, persistent, sz, A, ipiv, info, s);
+            return launch_status();
+        }
         return getrf_cluster(wl, bound, persistent, sz, max_m, A, ipiv, info, s);
     } else {
         if (max_m <= 128) launch_getrf_blocked<T, 32, 128, 128, 16>(wl, bound, persistent, sz, A, ipiv, info, s);
@@ -105,9 +131,9 @@ magma_int_t getrs_blocked(const WorkList& wl, int bound, bool persistent, bool t
     }
 }
 
-template magma_int_t getrf_blocked<double>(const WorkList&, int, bool, const LuSizes&, int, double**, int**, int*,
+template magma_int_t getrf_blocked<double>(const WorkList&, int, bool, const LuSizes&, int, int, double**, int**, int*,
                                            cudaStream_t);
-template magma_int_t getrf_blocked<float>(const WorkList&, int, bool, const LuSizes&, int, float**, int**, int*,
+template magma_int_t getrf_blocked<float>(const WorkList&, int, bool, const LuSizes&, int, int, float**, int**, int*,
                                           cudaStream_t);
 template magma_int_t getrs_blocked<double>(const WorkList&, int, bool, bool, const LuSizes&, int, int, double**, int**,
                                            double**, cudaStream_t);

@@ -29,7 +29,7 @@ magma_int_t getrf_impl(const char* name, magma_int_t m, magma_int_t n, T** dA_ar
     if (small_lu_supported(m, n))
         return getrf_small<T>(wl, batchCount, false, sz, m, n, dA_array, ipiv_array, info_array, queue->stream);
     if (blocked_lu_supported(m))
-        return getrf_blocked<T>(wl, batchCount, false, sz, m, dA_array, ipiv_array, info_array, queue->stream);
+        return getrf_blocked<T>(wl, batchCount, false, sz, m, n, dA_array, ipiv_array, info_array, queue->stream);
     return MAGMA_ERR_NOT_SUPPORTED;
 }
 

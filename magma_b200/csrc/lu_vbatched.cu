@@ -28,9 +28,9 @@ enum class LuOp { Getrf, Getrs, Gesv };
 
 template <typename T>
 static magma_int_t lu_var(LuOp op, bool trans, const int* m, const int* n, const int* nrhs, T** A, const int* lda,
-                          int** ipiv, T** B, const int* ldb, int* info, int batch, int max_mn, int max_nrhs,
+                          int** ipiv, T** B, const int* ldb, int* info, int batch, int max_m, int max_n, int max_nrhs,
                           magma_queue_t queue) {
-    const int top = lu_bucket_of(max_mn);
+    const int top = lu_bucket_of(std::max(max_m, max_n));
     if (top < 0) return MAGMA_ERR_NOT_SUPPORTED;
     const size_t bw = bucketize_ws_ints(batch, kLuBuckets);
     int* ws = static_cast<int*>(queue_workspace(queue, sizeof(int) * (bw + bucket_sort_ws_ints(batch, kLuBuckets))));
@@ -58,7 +58,7 @@ static magma_int_t lu_var(LuOp op, bool trans, const int* m, const int* n, const
             const int b = kLuBuckets - 1;
             const WorkList wl{lists + (size_t)b * batch, counts + b, 0};
             cudaStream_t s0 = queue_aux(queue, 0);
-            rc = getrf_blocked<T>(wl, batch, true, sz, kLuEdges[b], A, ipiv, info, s0);
+            rc = getrf_blocked<T>(wl, batch, true, sz, kLuEdges[b], std::min(max_n, kLuEdges[b]), A, ipiv, info, s0);
             if (!rc && solve) rc = getrs_blocked<T>(wl, batch, true, false, sz, kLuEdges[b], max_nrhs, A, ipiv, B, s0);
             lu_queue<T>(solve, counts, lists, batch, top, head, sz, A, ipiv, B, info, max_nrhs, queue_aux(queue, 1));
             queue_join(queue);
@@ -76,7 +76,7 @@ static magma_int_t lu_var(LuOp op, bool trans, const int* m, const int* n, const
             else if (op == LuOp::Gesv) rc = gesv_small<T>(wl, batch, true, sz, e, max_nrhs, A, ipiv, B, info, s);
             else rc = getrs_small<T>(wl, batch, true, trans, sz, e, max_nrhs, A, ipiv, B, s);
         } else {
-            if (op != LuOp::Getrs) rc = getrf_blocked<T>(wl, batch, true, sz, e, A, ipiv, info, s);
+            if (op != LuOp::Getrs) rc = getrf_blocked<T>(wl, batch, true, sz, e, std::min(max_n, e), A, ipiv, info, s);
             if (!rc && op != LuOp::Getrf)
                 rc = getrs_blocked<T>(wl, batch, true, trans, sz, e, max_nrhs, A, ipiv, B, s);
         }
@@ -112,7 +112,7 @@ magma_int_t magma_dgetrf_vbatched_max_nocheck(magma_int_t* m, magma_int_t* n, do
         return 0;
     }
     return lu_var<double>(LuOp::Getrf, false, m, n, nullptr, dA_array, ldda, ipiv_array, nullptr, nullptr, info_array,
-                          batchCount, std::max(max_m, max_n), 1, queue);
+                          batchCount, max_m, max_n, 1, queue);
 }
 
 // Checks: m -1, n -2, ldda < m -4, batchCount -7 (magma_zgetrf_batched's numbering).
@@ -144,7 +144,7 @@ magma_int_t magma_dgetrs_vbatched_max_nocheck(magma_trans_t trans, magma_int_t* 
                                               magma_int_t max_n, magma_int_t max_nrhs, magma_queue_t queue) {
     if (batchCount <= 0 || max_n <= 0 || max_nrhs <= 0) return 0;
     return lu_var<double>(LuOp::Getrs, trans != MagmaNoTrans, n, n, nrhs, dA_array, ldda, dipiv_array, dB_array, lddb,
-                          nullptr, batchCount, max_n, max_nrhs, queue);
+                          nullptr, batchCount, max_n, max_n, max_nrhs, queue);
 }
 
 // Checks: trans -1, n -2, nrhs -3, ldda < n -5, lddb < n -8, batchCount -10.
@@ -183,7 +183,7 @@ magma_int_t magma_dgesv_vbatched_max_nocheck(magma_int_t* n, magma_int_t* nrhs, 
         return 0;
     }
     return lu_var<double>(LuOp::Gesv, false, n, n, nrhs, dA_array, ldda, dipiv_array, dB_array, lddb, dinfo_array,
-                          batchCount, max_n, max_nrhs, queue);
+                          batchCount, max_n, max_n, max_nrhs, queue);
 }
 
 // Checks: n -1, nrhs -2, ldda < n -4, lddb < n -7, batchCount -9.

@@ -290,7 +290,7 @@ magma_int_t dsgesv_batched(int n, int nrhs, double** dA, int lda, int** ipiv, do
         const WorkList all{nullptr, nullptr, batch};
         const LuSizes szs{n, n, n, n, R, nullptr, nullptr, nullptr, nullptr, nullptr};
         rc = small_lu_supported(n, n) ? getrf_small<float>(all, batch, false, szs, n, n, w.SA_ptr, ipiv, w.sinfo, s)
-                                      : getrf_blocked<float>(all, batch, false, szs, n, w.SA_ptr, ipiv, w.sinfo, s);
+                                      : getrf_blocked<float>(all, batch, false, szs, n, n, w.SA_ptr, ipiv, w.sinfo, s);
         if (rc) return rc;
     }
     queue_stage_mark(queue);
@@ -307,7 +307,7 @@ magma_int_t dsgesv_batched(int n, int nrhs, double** dA, int lda, int** ipiv, do
     const WorkList failed{w.fail_list, w.fail_count, 0};
     const LuSizes szd{n, n, lda, ldx, nrhs, nullptr, nullptr, nullptr, nullptr, nullptr};
     rc = small_lu_supported(n, n) ? getrf_small<double>(failed, batch, true, szd, n, n, dA, ipiv, info, s)
-                                  : getrf_blocked<double>(failed, batch, true, szd, n, dA, ipiv, info, s);
+                                  : getrf_blocked<double>(failed, batch, true, szd, n, n, dA, ipiv, info, s);
     if (rc) return rc;
     copy_rhs_kernel<<<std::min(batch, 1184), 256, 0, s>>>(failed, n, nrhs, dB, ldb, dX, ldx);
     rc = small_lu_supported(n, n) ? getrs_small<double>(failed, batch, true, false, szd, n, nrhs, dA, ipiv, dX, s)

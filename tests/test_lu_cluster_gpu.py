@@ -57,19 +57,55 @@ def test_getrf_nopiv_cluster_bit_identical(cuda, m):
     assert np.array_equal(D.cpu().numpy(), O)
 
 
-@pytest.mark.parametrize("m,n", [(257, 1), (400, 2), (513, 1), (1024, 3)])
-def test_short_factorisations(cuda, m, n):
-    """A panel of one to three steps in more clusters than the machine holds at once: each cluster's
-    first exchange comes right after it starts, while its blocks replace other clusters'."""
+def _random_bit_identical(cuda, m, n, batch):
     import torch
 
     import magma_b200 as mb
     import oracle
-    A = np.random.default_rng(m).uniform(-1, 1, (1500, n, m))
+    A = np.random.default_rng(m + n).uniform(-1, 1, (batch, n, m))
     O = A.copy()
     oip, oinf = oracle.dgetrf_batched(O, m)
     D = torch.from_numpy(A).to(cuda)
     ipiv, info = mb.dgetrf_batched(D, m=m)
-    assert np.array_equal(ipiv.cpu().numpy()[:, :n], oip[:, :n])
+    k = min(m, n)
+    assert np.array_equal(ipiv.cpu().numpy()[:, :k], oip[:, :k])
     assert np.array_equal(info.cpu().numpy(), oinf)
     assert np.array_equal(D.cpu().numpy(), O)
+
+
+@pytest.mark.parametrize("m,n,batch", [(700, 17, 74), (1024, 20, 60), (600, 129, 300), (260, 161, 400)])
+def test_many_clusters(cuda, m, n, batch):
+    """Short factorisations in as many clusters as the machine holds at once, and more: a cluster's
+    first exchange comes right after it starts, while its blocks replace other clusters'."""
+    _random_bit_identical(cuda, m, n, batch)
+
+
+@pytest.mark.parametrize("m,few,many", [(257, 96, 160), (512, 96, 160), (513, 16, 128), (1024, 16, 128)])
+@pytest.mark.parametrize("past", [0, 1])
+def test_tall_rule(cuda, m, few, many, past):
+    """Matrices on both sides of the lines between the block and the cluster kernel, for few and for
+    many matrices; and the fewest columns."""
+    _random_bit_identical(cuda, m, few + past, 5)
+    _random_bit_identical(cuda, m, many + past, 80)
+    _random_bit_identical(cuda, m, 1 + past, 80)
+
+
+@pytest.mark.parametrize("cols", [40, 300])
+def test_tall_vbatched(cuda, cols):
+    """Variable sizes with tall instances, under a maximum of few and of many columns."""
+    import magma_b200 as mb
+    import oracle
+    from magma_b200.api import VarBatch
+    rng = np.random.default_rng(cols)
+    m = np.array([300, 512, 257, 513, 1024, 700, 40, 256, 128, 1000] * 9)
+    n = np.minimum(rng.integers(1, cols + 1, len(m)), np.where(m > 256, cols, 64))
+    n[3] = cols
+    As = [rng.uniform(-1, 1, (c, r)) for r, c in zip(m, n)]
+    gA = VarBatch(As, cuda)
+    ipiv, info = mb.dgesv_vbatched(gA, None, n, m=m, solve=False, max_sizes=(1024, cols))
+    ip = ipiv.cpu().numpy()
+    assert not info.cpu().numpy().any()
+    for i, out in enumerate(gA.unpack()):
+        O = As[i].copy()[None]
+        oip, _ = oracle.dgetrf_batched(O, int(m[i]))
+        assert np.array_equal(out, O[0]) and np.array_equal(ip[i, :oip.shape[1]], oip[0]), (m[i], n[i])
