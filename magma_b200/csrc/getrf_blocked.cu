@@ -1,6 +1,7 @@
 // getrf_blocked.cu -- kernels and host dispatch of the blocked batched LU
-// (one matrix per thread block, up to 1024 rows): FP32, and FP64 where a matrix is tall
-// (getrf_tall). Other FP64 calls run getrf_cluster.cu and getrs_tc.cu.
+// (one matrix per thread block, up to 1024 rows): FP32, and in FP64 the factors of tall matrices
+// (getrf_tall) and many solves of one right-hand side. Other FP64 calls run getrf_cluster.cu and
+// getrs_tc.cu.
 #include "internal.h"
 #include "blocked_lu.cuh"
 #include "getrs_blocked.cuh"
@@ -121,6 +122,17 @@ template <typename T>
 magma_int_t getrs_blocked(const WorkList& wl, int bound, bool persistent, bool trans, const LuSizes& sz, int max_n,
                           int max_nrhs, T** A, int** ipiv, T** B, cudaStream_t s) {
     if constexpr (std::is_same<T, double>::value) {
+        // One right-hand side fills one of the sweeps' eight columns. That costs nothing while every
+        // matrix has its block at once, which is up to five an SM; more matrices of one right-hand
+        // side are through sooner with a thread per row (n = 65 and 128, this form against the
+        // sweeps: 740 matrices 78 against 50 us and 118 against 81; 900, 77 against 80 and 124
+        // against 146; 2,000, 81 against 129 and 148 against 211; above 128 rows the sweeps win,
+        // 2,000 x 140^2 326 against 287).
+        if (max_nrhs <= 1 && max_n <= 128 && bound > 5 * device_sm_count()) {
+            auto k = getrs_blocked_kernel<T, 128, 1>;
+            k<<<blocked_grid(k, 128, bound, persistent), 128, 0, s>>>(wl, sz, trans, A, ipiv, B);
+            return launch_status();
+        }
         return getrs_tc(wl, bound, persistent, trans, sz, max_n, max_nrhs, A, ipiv, B, s);
     } else {
         if (max_n <= 128) launch_getrs_blocked<T, 128>(wl, bound, persistent, sz, trans, max_nrhs, A, ipiv, B, s);

@@ -53,3 +53,28 @@ def test_getrs_trans(cuda, n, nrhs):
     # each solution carries the backward error of two n-term substitutions, amplified by cond(A);
     # the oracle sums in another order: 64 n eps of the largest entry, as for the smaller orders
     assert np.abs(got - X).max() <= 64 * n * np.finfo(float).eps * np.abs(X).max()
+
+
+@pytest.mark.parametrize("n", [65, 128])
+@pytest.mark.parametrize("past", [0, 1])
+def test_one_rhs_many(cuda, n, past):
+    """One right-hand side on both sides of the line of five matrices an SM: the oracle's solutions,
+    and with trans the bits of the same solve beside a second right-hand side (always the sweeps)."""
+    import torch
+
+    import magma_b200 as mb
+    import oracle
+    batch = 5 * torch.cuda.get_device_properties(0).multi_processor_count + past
+    rng = np.random.default_rng(n + past)
+    A, B = rng.uniform(-1, 1, (batch, n, n)), rng.uniform(-1, 1, (batch, 2, n))
+    ipiv, _ = oracle.dgetrf_batched(A, n)
+    X = B[:, :1].copy()
+    oracle.dgetrs_batched(A, ipiv, X)
+    dA, dP = torch.from_numpy(A).to(cuda), torch.from_numpy(ipiv).to(cuda)
+    for trans in (False, True):
+        one, two = torch.from_numpy(B[:, :1].copy()).to(cuda), torch.from_numpy(B).to(cuda)
+        mb.dgetrs_batched(dA, dP, one, trans=trans)
+        mb.dgetrs_batched(dA, dP, two, trans=trans)
+        assert torch.equal(one, two[:, :1])
+        if not trans:
+            assert np.array_equal(one.cpu().numpy(), X)
