@@ -637,7 +637,8 @@ static magma_int_t gemm_launch_tc(bool TA, bool TB, const GemmSizes& g, T alpha,
 // flight, the same fragments, k-steps and epilogue as gemm_dmma_kernel, so the same bits. A is
 // staged by columns (rows padded to 68 doubles), B by its own columns (16 values of k, padded to
 // 20): both copies run along the contiguous direction, 16 bytes at a time where the instance's
-// pointer and leading dimension allow it, and both fragments touch every bank once. What lies
+// pointer and leading dimension allow it (8 otherwise, as many copies in flight: 2,000 x 128^3 with
+// odd leading dimensions 443 -> 371 us), and both fragments touch every bank once. What lies
 // outside the instance costs nothing: 8x8 sub-tiles past M or N take no MMA and no copy, k-steps
 // past K neither (a whole 64x64 tile is twice the work of an average C of orders 8..128). C's
 // lines are prefetched to L2 at the start. What bounds it: latency at three 4-warp blocks an SM
@@ -706,12 +707,15 @@ gemm_dmma_async_kernel(GemmSizes g, double alpha, const double* const* __restric
                 src += (size_t)(NT / 32) * lda;
             }
         } else {
-            for (int e = tid; e < 64 * kl; e += NT) {
-                const int r = e & 63, c = e >> 6;
-                if (r < mlive) {
-                    const bool v = (i0 + r < m) && (k0 + c < k);
-                    cp_async_elem(&sm.a[st][c][r], v ? A + (i0 + r) + (size_t)(k0 + c) * lda : A, v, 8);
-                }
+            const int r = tid & 63;
+            const bool in = i0 + r < m;
+            const double* src = A + i0 + r + (size_t)(k0 + (tid >> 6)) * lda;
+#pragma unroll
+            for (int e = 0; e < 64 * BK / NT; ++e) {
+                const int c = (tid >> 6) + e * (NT / 64);
+                const bool v = in && k0 + c < k;
+                if (r < mlive && c < kl) cp_async_elem(&sm.a[st][c][r], v ? src : A, v, 8);
+                src += (size_t)(NT / 64) * lda;
             }
         }
         if (vb) {   // two k's at a time
@@ -724,12 +728,15 @@ gemm_dmma_async_kernel(GemmSizes g, double alpha, const double* const* __restric
                 src += (size_t)(NT / 8) * ldb;
             }
         } else {
-            for (int e = tid; e < 16 * nlive; e += NT) {
-                const int c = e & 15, j = e >> 4;
-                if (c < kl) {
-                    const bool v = (k0 + c < k) && (j0 + j < n);
-                    cp_async_elem(&sm.b[st][j][c], v ? B + (k0 + c) + (size_t)(j0 + j) * ldb : B, v, 8);
-                }
+            const int c = tid & 15;
+            const bool in = k0 + c < k;
+            const double* src = B + k0 + c + (size_t)(j0 + (tid >> 4)) * ldb;
+#pragma unroll
+            for (int e = 0; e < 16 * BN / NT; ++e) {
+                const int j = (tid >> 4) + e * (NT / 16);
+                const bool v = in && j0 + j < n;
+                if (j < nlive && c < kl) cp_async_elem(&sm.b[st][j][c], v ? src : B, v, 8);
+                src += (size_t)(NT / 16) * ldb;
             }
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
