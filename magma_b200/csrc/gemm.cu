@@ -418,23 +418,39 @@ __device__ __forceinline__ int tc_kmajor(int row, int k) {   // float index of (
 
 // The first `left` of 32 consecutive values (zero past them), four a load where `vec` says that the
 // address allows it: a thread's row of an operand stored along k is one cache line, and one load
-// per value made each of a warp's loads touch 32 lines.
+// per value makes each of a warp's loads touch 32 lines. Whole rows, single loads and the last
+// chunk's rows have a loop each: with the choice inside every group of four the single loads lost
+// their overlap (2,000 x 128^3, A transposed, odd leading dimensions 356 -> 236 us, 64 x 512 x 300
+// 2,670 -> 1,702; aligned 64 x 512 x 300 1,185 -> 1,068).
 __device__ __forceinline__ void tc_load_k(float (&x)[kTcGemmKc], const float* p, int left, bool vec) {
+    if (vec && left >= kTcGemmKc) {
 #pragma unroll
-    for (int q = 0; q < kTcGemmKc; q += 4) {
-        float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        if (vec && q + 4 <= left) {
-            v = *reinterpret_cast<const float4*>(p + q);
-        } else {
-            if (q < left) v.x = p[q];
-            if (q + 1 < left) v.y = p[q + 1];
-            if (q + 2 < left) v.z = p[q + 2];
-            if (q + 3 < left) v.w = p[q + 3];
+        for (int q = 0; q < kTcGemmKc; q += 4) {
+            const float4 v = *reinterpret_cast<const float4*>(p + q);
+            x[q] = v.x;
+            x[q + 1] = v.y;
+            x[q + 2] = v.z;
+            x[q + 3] = v.w;
         }
-        x[q] = v.x;
-        x[q + 1] = v.y;
-        x[q + 2] = v.z;
-        x[q + 3] = v.w;
+    } else if (!vec) {
+#pragma unroll
+        for (int q = 0; q < kTcGemmKc; ++q) x[q] = q < left ? p[q] : 0.0f;
+    } else {
+#pragma unroll
+        for (int q = 0; q < kTcGemmKc; q += 4) {
+            float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            if (q + 4 <= left) {
+                v = *reinterpret_cast<const float4*>(p + q);
+            } else {
+                if (q < left) v.x = p[q];
+                if (q + 1 < left) v.y = p[q + 1];
+                if (q + 2 < left) v.z = p[q + 2];
+            }
+            x[q] = v.x;
+            x[q + 1] = v.y;
+            x[q + 2] = v.z;
+            x[q + 3] = v.w;
+        }
     }
 }
 

@@ -135,3 +135,35 @@ def test_syrk_vbatched_fp32_tensor_core(cuda, fp32_tensor_core_tile, lower):
         assert np.array_equal(got[~mask], c0[~mask].astype(np.float32).astype(np.float64)), i   # other triangle untouched
         den = np.sqrt(k + 2) * abs(alpha) * np.linalg.norm(op) ** 2 + 2 * abs(beta) * np.linalg.norm(c0)
         assert np.linalg.norm(np.where(mask, got - ref, 0)) / max(den, 1e-300) < 30 * eps, i
+
+
+@pytest.mark.parametrize("ta,tb", [(False, False), (True, False), (True, True)])
+@pytest.mark.parametrize("m,n,k", [(65, 70, 31), (128, 128, 32), (100, 33, 33), (130, 66, 67)])
+def test_alignment_does_not_matter(cuda, fp32_tensor_core_tile, ta, tb, m, n, k):
+    """Operands that allow 16-byte loads and the same operands with an odd leading dimension, or that
+    start on 4 bytes: the same bits, for whole and for cut chunks of 32 along k."""
+    import torch
+
+    import magma_b200 as mb
+    g = torch.Generator().manual_seed(m * 131 + k)
+    batch = 3
+    ra, ca, rb, cb = (k, m, n, k) if ta and tb else (k, m, k, n) if ta else (m, k, k, n)
+    A, B = (torch.randn(batch, c, r, generator=g).to(cuda) for r, c in ((ra, ca), (rb, cb)))
+
+    def place(M, ld, shift):
+        buf = torch.full((batch * M.shape[1] * ld + 4,), float("nan"), device=cuda)
+        out = buf[shift:shift + batch * M.shape[1] * ld].view(batch, M.shape[1], ld)
+        out[:, :, :M.shape[2]] = M
+        return out
+    results = []
+    for pad, shift in ((4, 0), (4, 1), (5, 0), (3, 2)):
+        out = torch.zeros(batch, n, m, device=cuda)
+        lda, ldb = (ra + 3) // 4 * 4 + pad, (rb + 3) // 4 * 4 + pad
+        mb.gemm_batched(place(A, lda, shift), place(B, ldb, shift), out, m, n, k, transA=ta, transB=tb)
+        results.append(out)
+    assert all(torch.equal(results[0], r) for r in results[1:])
+    ref = (A.double() if ta else A.double().transpose(1, 2)) @ (B.double() if tb else B.double().transpose(1, 2))
+    got = results[0].transpose(1, 2).double()
+    # the tester's bound, as above
+    den = np.sqrt(k + 2) * A.double().flatten(1).norm(dim=1) * B.double().flatten(1).norm(dim=1)
+    assert ((got - ref).flatten(1).norm(dim=1) / den).max().item() < 30 * np.finfo(np.float32).eps
