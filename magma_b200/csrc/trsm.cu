@@ -201,7 +201,7 @@ tri_panel_kernel(TriArgs<T> g, int panels, int batch) {
     }
 }
 
-// FP64 trsm of triangles up to kTrsmWarpRows rows: a warp takes eight columns of X from the first
+// FP64 trsm of triangles up to trsm_warp_rows rows: a warp takes eight columns of X from the first
 // row to the last and never meets another warp. Eight rows at a time (the MMA's accumulator: lane
 // l holds row l/4, columns 2(l%4), +1) it applies the rows already solved -- A fragments straight
 // from T, two batches of eight k-steps in flight, B fragments from the solved rows in shared
@@ -210,9 +210,16 @@ tri_panel_kernel(TriArgs<T> g, int panels, int batch) {
 // MMA applies its products in ascending k, each rounded): the same bits.
 // What bounds it: at 20 warps an SM, the dependent MMAs of a column group (29 cycles each) and the
 // loads of T. 20,000 triangles of 8..128 rows, 8..128 columns, with B's restore: 2,754 -> 1,979 us.
-// Above 256 rows the solved rows no longer leave room for enough warps and the panel
-// kernel stays.
-constexpr int kTrsmWarpRows = 256, kTrsmWarps = 4;
+constexpr int kTrsmWarps = 4;
+
+// The rows up to which the warp kernel takes a call; the panel kernel takes the rest. The solved rows
+// of 176 leave room for five blocks an SM. Past them the panel kernel is as fast or faster whatever
+// the columns (warp against panel kernel, 2,000 triangles: 176 rows, 1, 32 and 200 columns 0.67, 0.77
+// and 0.92 of its time; 192 rows 0.97, 1.03 and 1.21; 256 rows 1.37, 1.37 and 1.67). From the left
+// with a transposed T the panel kernel's reads of T cost more: one panel of columns wins up to 224
+// rows (224 rows, 1 and 32 columns 0.82 and 0.88; 256 rows 1.03 and 1.07), several do not (300
+// triangles of 224 rows, 33 and 64 columns 1.14 and 1.20).
+static int trsm_warp_rows(bool tt, bool bt, int panels) { return tt && !bt && panels == 1 ? 224 : 176; }
 
 __global__ void __launch_bounds__(32 * kTrsmWarps, 5)
 trsm_warp_kernel(TriArgs<double> g, bool flip, bool tt, bool bt, int panels, int rows) {
@@ -299,7 +306,7 @@ static bool trsm_warp(const TriArgs<T>& g, bool flip, bool tt, bool bt, int max_
                       cudaStream_t s) {
     if constexpr (std::is_same<T, double>::value) {
         static_assert(8 * kTrsmWarps == kTriTile, "a block's columns are a panel");
-        if (max_rows > kTrsmWarpRows) return false;
+        if (max_rows > trsm_warp_rows(tt, bt, panels)) return false;
         const int rows = (max_rows + 7) / 8 * 8;
         const int smem = (int)sizeof(double) * kTrsmWarps * rows * kTriRhs;
         ensure_dynamic_smem((const void*)trsm_warp_kernel, smem);
