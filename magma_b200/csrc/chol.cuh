@@ -266,18 +266,18 @@ __device__ __forceinline__ void potrs_small_instance(int id, const LuSizes& sz, 
 }
 
 // ---------------------------------------------------------------------------
-// Blocked right-looking Cholesky of one matrix per thread block (n <= NT): FP32, and FP64
-// above order 512 (smaller FP64 orders: chol_team.cuh).
+// Blocked right-looking FP64 Cholesky of one matrix per thread block (n <= NT): orders above 512
+// (smaller ones: chol_team.cuh).
 // Per panel of NB columns: thread t factors row t's panel entries in registers
 // (chol_panel_steps), every row publishes them to shared memory, and the
-// trailing lower triangle A22 -= P P^T is computed by all threads in 4x8 tiles
+// trailing lower triangle A22 -= P P^T is computed on the tensor cores in jobs
 // distributed evenly over the triangle (a row-per-thread update would leave
 // the last rows with most of the work). Each element still receives
 // fma(-L(i,r), L(j,r), a) for r ascending, the unblocked order.
-template <typename T, int NB, int NT, int CW>
+template <int NB, int NT>
 struct BlockedCholShared {
-    CholShared<T, NB> p;
-    T P[NT][NB + 1];     // panel entries of every row
+    CholShared<double, NB> p;
+    double P[NT][NB + 1];     // panel entries of every row
 };
 
 // One FP64 tensor-core step D = A B + D on an 8x8 tile (mma.sync m8n8k4: lane l holds
@@ -292,16 +292,14 @@ __device__ __forceinline__ void chol_dmma(double& d0, double& d1, double a, doub
 // Trailing update of one panel on the FP64 tensor cores: A22 -= P P^T on the lower
 // triangle from row/column m0 on, in jobs of 32 rows x 8 columns per warp (four 8x8
 // accumulator tiles, so four independent MMA chains). The multipliers come from the
-// panel rows in shared memory (A fragment negated: (-l_i) l_j + a is the fma of the
-// CUDA-core update), steps past the panel's nbp are zero, and each element receives its
-// nbp updates in ascending order, exactly as in the CUDA-core update. The next job's entries
-// are loaded before the current job's products.
-template <int NB, int NT, int CW, typename Team>
+// panel rows in shared memory (A fragment negated: (-l_i) l_j + a), steps past the panel's nbp
+// are zero, and each element receives its nbp updates in ascending order. The next job's
+// entries are loaded before the current job's products.
+template <int NB, int NT>
 __device__ __forceinline__ void chol_update_dmma(double* __restrict__ A, int n, int lda, bool upper, int m0,
-                                                 int nbp, const BlockedCholShared<double, NB, NT, CW>& sh,
-                                                 const Team& team) {
+                                                 int nbp, const BlockedCholShared<NB, NT>& sh) {
     constexpr int NW = NT / 32;
-    const int tid = team.tid(), lane = tid & 31, warp = tid >> 5;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int q = lane & 3, r8 = lane >> 2;
     const int T8 = (n - m0 + 7) / 8;   // 8-column tiles of the trailing triangle
     // element (i, j) of the stored triangle at A + i * si + j * sj (lower: A(i, j); upper: A(j, i))
@@ -368,22 +366,19 @@ __device__ __forceinline__ void chol_update_dmma(double* __restrict__ A, int n, 
     }
 }
 
-template <typename T, int NB, int NT, int CW, int CB, typename Team = BlockTeam, bool DMMA = false>
-__device__ int blocked_potrf(T* __restrict__ A, int n, int lda, bool upper, BlockedCholShared<T, NB, NT, CW>& sh,
-                             const Team& team = Team{}) {
+template <int NB, int NT>
+__device__ int blocked_potrf(double* __restrict__ A, int n, int lda, bool upper, BlockedCholShared<NB, NT>& sh) {
     constexpr int NW = NT / 32;
-    // tile rows x columns; 2 rows when the block size leaves 64 registers a thread (FP64)
-    constexpr int TR = (NT >= 1024 && sizeof(T) == 8) ? 2 : 4, TC = 8, G = 8 / TR;
-    const int tid = team.tid();
-    auto sync = [&] { team.sync(); };
+    const int tid = threadIdx.x;
+    auto sync = [] { __syncthreads(); };
     for (int k0 = 0; k0 < n; k0 += NB) {
         const int nbp = min(NB, n - k0);
         const bool live = (tid >= k0 && tid < n);
-        T a[NB];
+        double a[NB];
 #pragma unroll
         for (int c = 0; c < NB; ++c)
-            a[c] = (live && c < nbp && k0 + c <= tid) ? tri(A, lda, upper, tid, k0 + c) : T(0);
-        const int info = chol_panel_steps_unrolled<T, NB, NW>(a, n, nbp, k0, tid, sh.p, sync);
+            a[c] = (live && c < nbp && k0 + c <= tid) ? tri(A, lda, upper, tid, k0 + c) : 0.0;
+        const int info = chol_panel_steps_unrolled<double, NB, NW>(a, n, nbp, k0, tid, sh.p, sync);
         if (live) {
 #pragma unroll
             for (int c = 0; c < NB; ++c)
@@ -392,151 +387,11 @@ __device__ int blocked_potrf(T* __restrict__ A, int n, int lda, bool upper, Bloc
             for (int c = 0; c < NB; ++c) sh.P[tid][c] = a[c];
         }
         if (info) return info;
-        team.sync();
-        // trailing lower triangle: rows/columns m0..n-1, square 8x8 blocks (bj <= bi),
-        // each split into G work items of TR rows
-        const int m0 = k0 + nbp;
-        if constexpr (DMMA && std::is_same<T, double>::value) {
-            chol_update_dmma<NB, NT, CW>(A, n, lda, upper, m0, nbp, sh, team);
-            team.sync();   // trailing entries visible before the next panel loads them
-            continue;
-        }
-        const int T8 = (n - m0 + 7) / 8;
-        const int items = G * T8 * (T8 + 1) / 2;
-        for (int w = tid; w < items; w += NT) {
-            const int blk = w / G, h = w % G;
-            int bi = (int)((sqrtf(8.0f * blk + 1.0f) - 1.0f) * 0.5f);
-            while ((bi + 1) * (bi + 2) / 2 <= blk) ++bi;
-            while (bi * (bi + 1) / 2 > blk) --bi;
-            const int bj = blk - bi * (bi + 1) / 2;
-            const int i0 = m0 + 8 * bi + TR * h, j0 = m0 + 8 * bj;
-            T acc[TR][TC];
-#pragma unroll
-            for (int ii = 0; ii < TR; ++ii)
-#pragma unroll
-                for (int jj = 0; jj < TC; ++jj) {
-                    const int i = i0 + ii, j = j0 + jj;
-                    acc[ii][jj] = (i < n && j <= i) ? tri(A, lda, upper, i, j) : T(0);
-                }
-            for (int r = 0; r < nbp; ++r) {
-                T li[TR], lj[TC];
-#pragma unroll
-                for (int ii = 0; ii < TR; ++ii) li[ii] = sh.P[min(i0 + ii, NT - 1)][r];
-#pragma unroll
-                for (int jj = 0; jj < TC; ++jj) lj[jj] = sh.P[min(j0 + jj, NT - 1)][r];
-#pragma unroll
-                for (int ii = 0; ii < TR; ++ii)
-#pragma unroll
-                    for (int jj = 0; jj < TC; ++jj) acc[ii][jj] = fma_rn(-li[ii], lj[jj], acc[ii][jj]);
-            }
-#pragma unroll
-            for (int ii = 0; ii < TR; ++ii)
-#pragma unroll
-                for (int jj = 0; jj < TC; ++jj) {
-                    const int i = i0 + ii, j = j0 + jj;
-                    if (i < n && j <= i) tri(A, lda, upper, i, j) = acc[ii][jj];
-                }
-        }
-        team.sync();   // trailing entries visible before the next panel loads them
+        __syncthreads();
+        chol_update_dmma(A, n, lda, upper, k0 + nbp, nbp, sh);
+        __syncthreads();   // trailing entries visible before the next panel loads them
     }
     return 0;
-}
-
-// Blocked L L^T x = b for one matrix per thread block (n <= NT), R RHS at a time.
-template <typename T, int NT, int R>
-struct BlockedCholRsShared {
-    T sb[32][R];
-    T D[32][33];
-    T rD[32];   // 1 / D(i,i) of the current diagonal block
-};
-
-// The warp that owns diagonal block [j0, j0+cnt) loads it into shared memory (rows past
-// cnt: zero) with its reciprocals: the loads go out unconditionally, clamped inside the
-// matrix, 8 at a time, so they overlap instead of completing one by one.
-template <typename T, int NT, int R, typename F>
-__device__ __forceinline__ void load_diag_block(BlockedCholRsShared<T, NT, R>& sh, int cnt, int lane, F&& Lb) {
-    const int li = min(lane, cnt - 1);
-#pragma unroll
-    for (int c0 = 0; c0 < 32; c0 += 8) {
-        T v[8];
-#pragma unroll
-        for (int c = 0; c < 8; ++c) v[c] = Lb(li, min(c0 + c, cnt - 1));
-#pragma unroll
-        for (int c = 0; c < 8; ++c)
-            if (c0 + c <= lane && lane < cnt) sh.D[lane][c0 + c] = v[c];
-    }
-    if (lane < cnt) sh.rD[lane] = T(1) / Lb(lane, lane);
-    __syncwarp();
-}
-
-template <typename T, int NT, int R, typename Team = BlockTeam>
-__device__ void blocked_potrs(const T* __restrict__ A, int n, int lda, bool upper, T* __restrict__ B, int nrhs,
-                              int ldb, BlockedCholRsShared<T, NT, R>& sh, const Team& team = Team{}) {
-    const int t = team.tid(), lane = t & 31;
-    const int nblk = (n + 31) / 32;
-    auto L = [&](int i, int j) -> T { return upper ? A[j + (size_t)i * lda] : A[i + (size_t)j * lda]; };
-    for (int c0 = 0; c0 < nrhs; c0 += R) {
-        T b[R];
-#pragma unroll
-        for (int r = 0; r < R; ++r) b[r] = (t < n && c0 + r < nrhs) ? B[t + (size_t)(c0 + r) * ldb] : T(0);
-        // forward: L y = b, blocks ascending
-        for (int J = 0; J < nblk; ++J) {
-            const int j0 = J * 32, j1 = min(n, j0 + 32), cnt = j1 - j0;
-            team.sync();
-            if ((t >> 5) == J) {
-                load_diag_block(sh, cnt, lane, [&](int i, int j) { return L(j0 + i, j0 + j); });
-                // steps unrolled over the block (no loop or branch overhead on the chain)
-                static_for<0, 32>([&](auto kc) {
-                    constexpr int k = decltype(kc)::value;
-                    if (k >= cnt) return;
-                    if (lane == k) {
-#pragma unroll
-                        for (int r = 0; r < R; ++r) { b[r] = b[r] * sh.rD[k]; sh.sb[k][r] = b[r]; }
-                    }
-                    __syncwarp();
-                    if (lane > k && lane < cnt) {
-                        const T l = sh.D[lane][k];
-#pragma unroll
-                        for (int r = 0; r < R; ++r) b[r] = fma_rn(-sh.sb[k][r], l, b[r]);
-                    }
-                });
-            }
-            team.sync();
-            if (t >= j1 && t < n)
-                block_update<T, R, false>(b, sh.sb, cnt, [&](int q) { return L(t, j0 + q); });
-        }
-        // backward: L^T x = y, blocks descending (column sweep of U = L^T)
-        for (int J = nblk - 1; J >= 0; --J) {
-            const int j0 = J * 32, j1 = min(n, j0 + 32), cnt = j1 - j0;
-            team.sync();
-            if ((t >> 5) == J) {
-                load_diag_block(sh, cnt, lane, [&](int i, int j) { return L(j0 + i, j0 + j); });
-                static_for<0, 32>([&](auto kc) {
-                    constexpr int k = 31 - decltype(kc)::value;
-                    if (k >= cnt) return;
-                    if (lane == k) {
-#pragma unroll
-                        for (int r = 0; r < R; ++r) { b[r] = b[r] * sh.rD[k]; sh.sb[k][r] = b[r]; }
-                    }
-                    __syncwarp();
-                    if (lane < k) {
-                        const T u = sh.D[k][lane];   // U(t, k) = L(k, t)
-#pragma unroll
-                        for (int r = 0; r < R; ++r) b[r] = fma_rn(-sh.sb[k][r], u, b[r]);
-                    }
-                });
-            }
-            team.sync();
-            if (t < j0)
-                block_update<T, R, true>(b, sh.sb, cnt, [&](int q) { return L(j0 + q, t); });
-        }
-        if (t < n) {
-#pragma unroll
-            for (int r = 0; r < R; ++r)
-                if (c0 + r < nrhs) B[t + (size_t)(c0 + r) * ldb] = b[r];
-        }
-        team.sync();
-    }
 }
 
 }  // namespace mb200

@@ -40,32 +40,18 @@ potrs_small_kernel(WorkList wl, LuSizes sz, bool upper, T** dA_array, T** dB_arr
     }
 }
 
-// ---- blocked potrf / potrs, one matrix per block ----
-template <typename T, int NB, int NT, int CW, int CB>
-__global__ void __launch_bounds__(NT, (NT <= 128 ? 4 : NT == 256 ? 2 : 1))
-potrf_blocked_kernel(WorkList wl, LuSizes sz, bool upper, T** dA_array, int* info_array) {
+// ---- blocked FP64 potrf (orders above 512), one matrix per block ----
+template <int NB, int NT>
+__global__ void __launch_bounds__(NT, 1)
+potrf_blocked_kernel(WorkList wl, LuSizes sz, bool upper, double** dA_array, int* info_array) {
     extern __shared__ __align__(16) unsigned char potrf_smem[];
-    BlockedCholShared<T, NB, NT, CW>& sh = *reinterpret_cast<BlockedCholShared<T, NB, NT, CW>*>(potrf_smem);
+    BlockedCholShared<NB, NT>& sh = *reinterpret_cast<BlockedCholShared<NB, NT>*>(potrf_smem);
     for (int w = blockIdx.x; w < wl.size(); w += gridDim.x) {
         const int id = wl.at(w);
         const int n = sz.get_n(id), lda = sz.get_lda(id);
         int info = 0;
-        // FP64: the trailing updates on the tensor cores (the same bits as the CUDA-core form)
-        if (n > 0) info = blocked_potrf<T, NB, NT, CW, CB, BlockTeam, std::is_same<T, double>::value>(
-                       dA_array[id], n, lda, upper, sh);
+        if (n > 0) info = blocked_potrf(dA_array[id], n, lda, upper, sh);
         if (threadIdx.x == 0 && info_array) info_array[id] = info;
-        __syncthreads();
-    }
-}
-
-template <typename T, int NT, int R>
-__global__ void __launch_bounds__(NT)
-potrs_blocked_kernel(WorkList wl, LuSizes sz, bool upper, T** dA_array, T** dB_array) {
-    __shared__ BlockedCholRsShared<T, NT, R> sh;
-    for (int w = blockIdx.x; w < wl.size(); w += gridDim.x) {
-        const int id = wl.at(w);
-        const int n = sz.get_n(id), lda = sz.get_lda(id), nrhs = sz.get_nrhs(id), ldb = sz.get_ldb(id);
-        if (n > 0 && nrhs > 0) blocked_potrs<T, NT, R>(dA_array[id], n, lda, upper, dB_array[id], nrhs, ldb, sh);
         __syncthreads();
     }
 }
@@ -111,18 +97,16 @@ static void launch_chol_small(const WorkList& wl, int bound, bool persistent, co
     constexpr int MPB = CholShape<NW>::MPB;
     const int threads = 32 * NW * MPB;
     const int items = ceildiv(bound, MPB);
-    if (!solve) {
-        auto k = chol_small_kernel<T, NC, NW, 1, false>;
+    auto launch = [&](auto k) {
         k<<<grid_for(k, threads, items, persistent), threads, 0, s>>>(wl, sz, upper, A, B, info);
-    } else if (max_nrhs <= 1) {
-        auto k = chol_small_kernel<T, NC, NW, 1, true>;
-        k<<<grid_for(k, threads, items, persistent), threads, 0, s>>>(wl, sz, upper, A, B, info);
-    } else if (max_nrhs <= 4) {
-        auto k = chol_small_kernel<T, NC, NW, 4, true>;
-        k<<<grid_for(k, threads, items, persistent), threads, 0, s>>>(wl, sz, upper, A, B, info);
+    };
+    if constexpr (std::is_same<T, float>::value) {   // the mixed solve's factor
+        launch(chol_small_kernel<T, NC, NW, 1, false>);
     } else {
-        auto k = chol_small_kernel<T, NC, NW, 8, true>;
-        k<<<grid_for(k, threads, items, persistent), threads, 0, s>>>(wl, sz, upper, A, B, info);
+        if (!solve) launch(chol_small_kernel<T, NC, NW, 1, false>);
+        else if (max_nrhs <= 1) launch(chol_small_kernel<T, NC, NW, 1, true>);
+        else if (max_nrhs <= 4) launch(chol_small_kernel<T, NC, NW, 4, true>);
+        else launch(chol_small_kernel<T, NC, NW, 8, true>);
     }
 }
 
@@ -144,62 +128,68 @@ static void launch_potrs_small(const WorkList& wl, int bound, bool persistent, c
     }
 }
 
-template <typename T, int NB, int NT, int CW, int CB>
+template <typename T, int S>
+static void launch_potrf_team(const WorkList& wl, int bound, bool persistent, const LuSizes& sz, bool upper, T** A,
+                              int* info, cudaStream_t s) {
+    auto k = potrf_team_kernel<T, S>;
+    const int smem = (int)(sizeof(T) == 8 ? chol_team_smem(S) : sizeof(T) * (32 * S + 32 * 33 + 32) + 16);
+    ensure_dynamic_smem((const void*)k, smem);
+    k<<<grid_for(k, S, bound, persistent, smem), S, smem, s>>>(wl, sz, upper, A, info);
+}
+
 static void launch_potrf_blocked(const WorkList& wl, int bound, bool persistent, const LuSizes& sz, bool upper,
-                                 T** A, int* info, cudaStream_t s) {
-    if constexpr (NT <= 512) {
-        auto k = potrf_team_kernel<T, NT>;
-        const int smem = (int)(sizeof(T) == 8 ? chol_team_smem(NT) : sizeof(T) * (32 * NT + 32 * 33 + 32) + 16);
-        ensure_dynamic_smem((const void*)k, smem);
-        k<<<grid_for(k, NT, bound, persistent, smem), NT, smem, s>>>(wl, sz, upper, A, info);
-        return;
-    }
-    auto k = potrf_blocked_kernel<T, NB, NT, CW, CB>;
-    const int smem = (int)sizeof(BlockedCholShared<T, NB, NT, CW>);
+                                 double** A, int* info, cudaStream_t s) {
+    constexpr int NB = 16, NT = 1024;
+    auto k = potrf_blocked_kernel<NB, NT>;
+    const int smem = (int)sizeof(BlockedCholShared<NB, NT>);
     ensure_dynamic_smem((const void*)k, smem);
     k<<<grid_for(k, NT, bound, persistent, smem), NT, smem, s>>>(wl, sz, upper, A, info);
 }
 
-template <typename T, int NT>
-static void launch_potrs_blocked(const WorkList& wl, int bound, bool persistent, const LuSizes& sz, bool upper,
-                                 T** A, T** B, int max_nrhs, cudaStream_t s) {
-    if constexpr (std::is_same<T, double>::value) {
-        constexpr int S = NT < 256 ? NT / 2 : NT == 256 ? 128 : 256;   // as the LU solves (getrs_tc.cu)
-        auto k = potrs_team_kernel<S, NT>;
-        const int smem = (int)(sizeof(double) * kTriRhs * NT + sizeof(TriStage));
-        ensure_dynamic_smem((const void*)k, smem);
-        const int gy = min(4, ceildiv(max(1, max_nrhs), kTriRhs));
-        k<<<dim3(grid_for(k, S, bound, persistent, smem), gy), S, smem, s>>>(wl, sz, upper, A, B);
-        return;
-    }
-    if (max_nrhs <= 1) {
-        auto k = potrs_blocked_kernel<T, NT, 1>;
-        k<<<grid_for(k, NT, bound, persistent), NT, 0, s>>>(wl, sz, upper, A, B);
-    } else if (max_nrhs <= 4) {
-        auto k = potrs_blocked_kernel<T, NT, 4>;
-        k<<<grid_for(k, NT, bound, persistent), NT, 0, s>>>(wl, sz, upper, A, B);
-    } else {
-        auto k = potrs_blocked_kernel<T, NT, 8>;
-        k<<<grid_for(k, NT, bound, persistent), NT, 0, s>>>(wl, sz, upper, A, B);
-    }
+// FP64 potrs of orders up to ROWS; threads as the LU solves (getrs_tc.cu).
+template <int ROWS>
+static void launch_potrs_team(const WorkList& wl, int bound, bool persistent, const LuSizes& sz, bool upper,
+                              double** A, double** B, int max_nrhs, cudaStream_t s) {
+    constexpr int S = ROWS < 256 ? ROWS / 2 : ROWS == 256 ? 128 : 256;
+    auto k = potrs_team_kernel<S, ROWS>;
+    const int smem = (int)(sizeof(double) * kTriRhs * ROWS + sizeof(TriStage));
+    ensure_dynamic_smem((const void*)k, smem);
+    const int gy = min(4, ceildiv(max(1, max_nrhs), kTriRhs));
+    k<<<dim3(grid_for(k, S, bound, persistent, smem), gy), S, smem, s>>>(wl, sz, upper, A, B);
 }
 
 // Size buckets shared by the Cholesky launchers (upper edges, inclusive).
 const int kCholEdges[kCholBuckets] = {8, 16, 32, 64, 128, 256, 512, 1024};
 
-template <typename T>
-void chol_bucket(int b, const WorkList& wl, int bound, bool persistent, const LuSizes& sz, bool upper, T** A, T** B,
-                 int* info, bool factor, bool solve, int max_nrhs, cudaStream_t s) {
+// FP32 is the mixed solve's factor: orders up to 512, no solve.
+template <>
+void chol_bucket<float>(int b, const WorkList& wl, int bound, bool persistent, const LuSizes& sz, bool upper, float** A,
+                        float** B, int* info, bool, bool, int, cudaStream_t s) {
+    switch (b) {
+        case 0: launch_chol_small<float, 8, 1>(wl, bound, persistent, sz, upper, A, B, info, false, 0, s); break;
+        case 1: launch_chol_small<float, 16, 1>(wl, bound, persistent, sz, upper, A, B, info, false, 0, s); break;
+        case 2: launch_chol_small<float, 32, 1>(wl, bound, persistent, sz, upper, A, B, info, false, 0, s); break;
+        case 3: launch_chol_small<float, 64, 2>(wl, bound, persistent, sz, upper, A, B, info, false, 0, s); break;
+        case 4: launch_potrf_team<float, 128>(wl, bound, persistent, sz, upper, A, info, s); break;
+        case 5: launch_potrf_team<float, 256>(wl, bound, persistent, sz, upper, A, info, s); break;
+        default: launch_potrf_team<float, 512>(wl, bound, persistent, sz, upper, A, info, s); break;
+    }
+}
+
+template <>
+void chol_bucket<double>(int b, const WorkList& wl, int bound, bool persistent, const LuSizes& sz, bool upper,
+                         double** A, double** B, int* info, bool factor, bool solve, int max_nrhs, cudaStream_t s) {
+    using T = double;
     if (factor) {
         switch (b) {
             case 0: launch_chol_small<T, 8, 1>(wl, bound, persistent, sz, upper, A, B, info, solve, max_nrhs, s); break;
             case 1: launch_chol_small<T, 16, 1>(wl, bound, persistent, sz, upper, A, B, info, solve, max_nrhs, s); break;
             case 2: launch_chol_small<T, 32, 1>(wl, bound, persistent, sz, upper, A, B, info, solve, max_nrhs, s); break;
             case 3: launch_chol_small<T, 64, 2>(wl, bound, persistent, sz, upper, A, B, info, solve, max_nrhs, s); break;
-            case 4: launch_potrf_blocked<T, 32, 128, 64, 8>(wl, bound, persistent, sz, upper, A, info, s); break;
-            case 5: launch_potrf_blocked<T, 32, 256, 64, 8>(wl, bound, persistent, sz, upper, A, info, s); break;
-            case 6: launch_potrf_blocked<T, 32, 512, 64, 8>(wl, bound, persistent, sz, upper, A, info, s); break;
-            default: launch_potrf_blocked<T, 16, 1024, 64, 4>(wl, bound, persistent, sz, upper, A, info, s); break;
+            case 4: launch_potrf_team<T, 128>(wl, bound, persistent, sz, upper, A, info, s); break;
+            case 5: launch_potrf_team<T, 256>(wl, bound, persistent, sz, upper, A, info, s); break;
+            case 6: launch_potrf_team<T, 512>(wl, bound, persistent, sz, upper, A, info, s); break;
+            default: launch_potrf_blocked(wl, bound, persistent, sz, upper, A, info, s); break;
         }
         if (!solve || b <= 3) return;   // small buckets fuse the solve into the factor kernel
     }
@@ -208,10 +198,10 @@ void chol_bucket(int b, const WorkList& wl, int bound, bool persistent, const Lu
         case 1: launch_potrs_small<T, 16, 1>(wl, bound, persistent, sz, upper, A, B, max_nrhs, s); break;
         case 2: launch_potrs_small<T, 32, 1>(wl, bound, persistent, sz, upper, A, B, max_nrhs, s); break;
         case 3: launch_potrs_small<T, 64, 2>(wl, bound, persistent, sz, upper, A, B, max_nrhs, s); break;
-        case 4: launch_potrs_blocked<T, 128>(wl, bound, persistent, sz, upper, A, B, max_nrhs, s); break;
-        case 5: launch_potrs_blocked<T, 256>(wl, bound, persistent, sz, upper, A, B, max_nrhs, s); break;
-        case 6: launch_potrs_blocked<T, 512>(wl, bound, persistent, sz, upper, A, B, max_nrhs, s); break;
-        default: launch_potrs_blocked<T, 1024>(wl, bound, persistent, sz, upper, A, B, max_nrhs, s); break;
+        case 4: launch_potrs_team<128>(wl, bound, persistent, sz, upper, A, B, max_nrhs, s); break;
+        case 5: launch_potrs_team<256>(wl, bound, persistent, sz, upper, A, B, max_nrhs, s); break;
+        case 6: launch_potrs_team<512>(wl, bound, persistent, sz, upper, A, B, max_nrhs, s); break;
+        default: launch_potrs_team<1024>(wl, bound, persistent, sz, upper, A, B, max_nrhs, s); break;
     }
 }
 
@@ -220,10 +210,5 @@ int chol_bucket_of(int n) {
         if (n <= kCholEdges[b]) return b;
     return -1;
 }
-
-template void chol_bucket<double>(int, const WorkList&, int, bool, const LuSizes&, bool, double**, double**, int*, bool,
-                                  bool, int, cudaStream_t);
-template void chol_bucket<float>(int, const WorkList&, int, bool, const LuSizes&, bool, float**, float**, int*, bool,
-                                 bool, int, cudaStream_t);
 
 }  // namespace mb200
