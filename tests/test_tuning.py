@@ -141,36 +141,41 @@ def test_autotune_runs(cuda, tmp_path):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("n", [100, 256, 300, 700])
-def test_lu_update_variants_bit_identical(cuda, n):
-    """The FP64 blocked LU's trailing update on the tensor cores (DMMA) and on the FP64
-    pipe give the same factors, pivots and info bit for bit, and both equal the oracle."""
-    import torch
-
+@pytest.mark.parametrize("n", [100, 256, 300, 512])
+def test_lu_queue_and_cluster_bit_identical(cuda, n):
+    """The FP64 LU's two live forms of the trailing update, on the FP64 pipe (the teams of the
+    one-launch variable-size LU, lu_queue = 1) and on the tensor cores (the cluster kernel,
+    lu_queue = 0), give the same factors, pivots and info bit for bit, and the oracle's. Values
+    9..12 of the table are not read: setting them changes nothing."""
     import magma_b200 as mb
     import oracle
     from magma_b200 import testing as T
+    from magma_b200.api import VarBatch
     lib = _lib.load()
     orig = _get(lib)
-    batch = max(2, 3_000_000 // (n * n))
+    batch = max(6, 3_000_000 // (n * n))
     A_np, _ = T.lu_uniform(batch, n, 1, seed=n)
     A_np[0, 7, :] = 0.0                      # a singular instance (zero column 8)
-    res = {}
+    ns = np.array([n - i % 3 for i in range(batch)], np.int32)   # three orders at the bucket's edge
+    mats = [np.ascontiguousarray(A_np[i, :k, :k]) for i, k in enumerate(ns)]
+    res = []
     try:
-        for v in (0, 1):
-            assert _set(lib, orig[:9] + [v] * 4 + orig[13:]) == 0
-            A = torch.from_numpy(A_np).to(cuda)
-            ipiv, info = mb.dgetrf_batched(A)
-            torch.cuda.synchronize()
-            res[v] = (A.cpu().numpy(), ipiv.cpu().numpy(), info.cpu().numpy())
+        for queue, unread in ((1, 0), (0, 0), (0, 1)):
+            assert _set(lib, orig[:9] + [unread] * 4 + orig[13:20] + [queue]) == 0
+            A = VarBatch(mats, cuda)
+            ipiv, info = mb.dgesv_vbatched(A, None, ns, solve=False, max_sizes=(n, n))
+            res.append((A.buf.cpu().numpy(), ipiv.cpu().numpy(), info.cpu().numpy()))
+            last = A.unpack()
     finally:
         _set(lib, orig)
-    for a, b in zip(res[0], res[1]):
-        assert np.array_equal(a, b)
-    O = A_np[:3].copy()
-    oip, oinf = oracle.dgetrf_batched(O, n)
-    assert np.array_equal(res[1][0][:3], O) and np.array_equal(res[1][1][:3], oip)
-    assert np.array_equal(res[1][2][:3], oinf) and oinf[0] == 8
+    for other in res[1:]:
+        for a, b in zip(res[0], other):
+            assert np.array_equal(a, b)
+    for i in range(6):
+        O = mats[i].copy()[None]
+        oip, oinf = oracle.dgetrf_batched(O, int(ns[i]))
+        assert np.array_equal(last[i], O[0]) and np.array_equal(res[2][1][i, :ns[i]], oip[0])
+        assert res[2][2][i] == oinf[0] == (8 if i == 0 else 0)
 
 
 @pytest.mark.gpu
