@@ -149,6 +149,14 @@ def dgesv_batched(A: np.ndarray, B: np.ndarray):
     return ipiv, info
 
 
+def spotrf(A: np.ndarray) -> int:
+    """Single-precision Cholesky of one column-major (n, n) array, lower, in place. Returns info."""
+    assert A.dtype == np.float32 and A.flags.c_contiguous
+    info = C.c_int()
+    lib().oracle_spotrf(A.shape[0], A.ctypes.data_as(_fp), A.shape[1], C.byref(info))
+    return info.value
+
+
 def dposv_vbatched(As, Bs, ns, nrhss, ldas, ldbs, solve=True, upper=False):
     """Restated Cholesky (+ solve) on lists of column-major arrays, in place. Returns info."""
     batch = len(As)

@@ -259,6 +259,22 @@ void oracle_dpotrf(int upper, int n, double* a, int lda, int* info) {
 #undef AL
 }
 
+/* The same factorisation in single precision, lower: the factor of the mixed solve
+ * (spotrf in the reference's src/zcposv_gpu.cpp:216). */
+void oracle_spotrf(int n, float* a, int lda, int* info) {
+    *info = 0;
+    for (int k = 0; k < n; ++k) {
+        float d = A_(k, k);
+        if (!(d > 0.0f)) { *info = k + 1; return; }
+        d = sqrtf(d);
+        A_(k, k) = d;
+        const float r = 1.0f / d;
+        for (int i = k + 1; i < n; ++i) A_(i, k) = A_(i, k) * r;
+        for (int j = k + 1; j < n; ++j)
+            for (int i = j; i < n; ++i) A_(i, j) = fmaf(-A_(i, k), A_(j, k), A_(i, j));
+    }
+}
+
 /* LAPACK dpotrs: L y = b (column sweep, reference DTRSM Left Lower NoTrans
  * NonUnit), then L^T x = y by the column sweep of the upper-triangular solve
  * with U = L^T (reference DTRSM Left Upper NoTrans NonUnit loop order), except

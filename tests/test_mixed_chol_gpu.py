@@ -100,6 +100,41 @@ def test_dsposv_vbatched_independent_of_the_batch(cuda):
             assert np.array_equal(X[i], results[0][0][i]), (i, ns[i])
 
 
+def test_single_precision_factor(cuda):
+    """The FP32 factor that the refinement solves with, left in the caller's workspace: the oracle's
+    bits at the edges of the 32-column panels and of the team sizes, at odd leading dimensions of A. A
+    wrong entry would otherwise cost passes only."""
+    import ctypes as C
+
+    import torch
+
+    from magma_b200.api import VarBatch, default_queue
+    ns = np.array([20, 33, 64, 65, 96, 97, 128, 129, 160, 255, 256, 257, 300, 480, 511, 512], np.int32)
+    batch, rng = len(ns), np.random.default_rng(12)
+    lda = ns + ns % 3
+    As = []
+    for i, n in enumerate(ns):
+        a = np.zeros((n, lda[i]))
+        a[:, :n] = T.spd_gram(int(n), 71, i)
+        As.append(a)
+    Bs = [rng.standard_normal((2, int(n))) for n in ns]
+    gA, gB, gX = VarBatch(As, cuda), VarBatch(Bs, cuda), VarBatch([np.zeros_like(b) for b in Bs], cuda)
+    gW = VarBatch([np.zeros((int(n) + 2, int(n))) for n in ns], cuda, torch.float32)
+    it, info = gA.ints(np.zeros(batch)), gA.ints(np.zeros(batch))
+    dn, dr, dla = gA.ints(ns), gA.ints(np.full(batch, 2)), gA.ints(lda)
+    q = default_queue()
+    p = lambda t: C.c_void_p(t.data_ptr())
+    rc = q.lib.magma_dsposv_vbatched_max_nocheck(122, p(dn), p(dr), p(gA.ptrs), p(dla), p(gB.ptrs), p(dn), p(gX.ptrs), p(dn),
+                                                 p(gW.ptrs), p(it), p(info), batch, 512, 2, q.handle)
+    q.sync()
+    assert rc == 0 and (it.cpu().numpy()[:batch] >= 0).all()
+    for i, (n, W) in enumerate(zip(ns, gW.unpack())):
+        ref = np.ascontiguousarray(As[i][:, :n]).astype(np.float32)
+        assert oracle.spotrf(ref) == 0
+        lower = np.triu(np.ones((n, n), bool))         # [column, row]
+        assert np.array_equal(W[:n][lower], ref[lower]), n
+
+
 def test_dsposv_vbatched_argument_errors(cuda):
     import magma_b200 as mb
     from magma_b200.api import VarBatch
