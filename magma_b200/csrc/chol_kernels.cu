@@ -57,6 +57,11 @@ potrf_blocked_kernel(WorkList wl, LuSizes sz, bool upper, double** dA_array, int
 }
 
 // ---- potrf (n <= S) and FP64 potrs (n <= ROWS) by a block of S threads ----
+// FP32: 768 threads an SM at 80 registers (228 bytes of spills), 1,024 at 64 for S = 512. Up to S =
+// 256 neither 512 threads (128 registers, 28 bytes) nor 1,024 (64, 304 bytes) change the mixed call by
+// more than 8% either way (1,000 orders 65..128, 1 RHS 361 us, 339 and 343; 10,000 of them 2,521,
+// 2,520 and 2,502). At S = 512, two blocks an SM against one: 1,000 orders 257..512, 1 RHS 4,937 us
+// and 5,000; 1,000 orders 4..512, 1 RHS, where other orders run beside them, 1,633 and 1,324.
 template <typename T, int S>
 __global__ void __launch_bounds__(S, (sizeof(T) == 4 ? (S == 512 ? 2 : 768 / S) : S <= 128 ? 4 : S == 256 ? 2 : 1))
 potrf_team_kernel(WorkList wl, LuSizes sz, bool upper, T** dA_array, int* info_array) {
@@ -154,7 +159,7 @@ static void launch_potrs_team(const WorkList& wl, int bound, bool persistent, co
     auto k = potrs_team_kernel<S, ROWS>;
     const int smem = (int)(sizeof(double) * kTriRhs * ROWS + sizeof(TriStage));
     ensure_dynamic_smem((const void*)k, smem);
-    const int gy = min(4, ceildiv(max(1, max_nrhs), kTriRhs));
+    const int gy = min(4, ceildiv(max(1, max_nrhs), kTriRhs));   // as the LU solves
     k<<<dim3(grid_for(k, S, bound, persistent, smem), gy), S, smem, s>>>(wl, sz, upper, A, B);
 }
 

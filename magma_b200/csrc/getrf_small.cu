@@ -19,7 +19,8 @@ MB200_SMALL_VARIANTS(MB200_DECLARE_SMALL)
 // Grid for a list of at most `bound` items handled MPB per block: one item per
 // block slot for a plain batch; for a device list (length unknown on the host)
 // the resident block count of the SMs, walked with a grid-stride loop: what the registers
-// are sized for (MinBlocks), one more for getrf alone of 32 columns (variable-size, 50,000 x 32^2 686 -> 548 us).
+// are sized for (MinBlocks), one more for getrf alone of 32 columns (variable-size,
+// 50,000 x 32^2 686 -> 548 us).
 static int small_grid(int nw, int nc, bool getrf, int bound, bool persistent) {
     const int mpb = (nw == 1) ? 4 : 1;
     const int items = ceildiv(bound, mpb);

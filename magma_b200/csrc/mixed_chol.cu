@@ -105,9 +105,10 @@ dlat2s_norm_vkernel(WorkList wl, const int* n_arr, double** dA_array, const int*
 // ---- 2. refinement of orders above kCholRowsMax: one block of NT threads per instance, n <= NMAX,
 // eight right-hand sides at a time. The correction solves L L^T c = r with the FP32 factor, widened,
 // in FP64 arithmetic on the tensor cores (tri_solve.cuh); the iteration counts are those of FP32
-// corrections (orders 129..512, 1 to 8 RHS, up to 1,000 instances: all equal). The residual B - A X is a tensor-core product over the stored triangle (a warp
-// per 16 rows). Both read A and L along their contiguous direction whichever triangle an element
-// lies in; the former thread-per-row loops read half of each with 32 lines a load.
+// corrections (orders 129..512, 1 to 8 RHS, up to 1,000 instances: all equal). The residual B - A X
+// is a tensor-core product over the stored triangle (a warp per 16 rows). Both read A and L along
+// their contiguous direction whichever triangle an element lies in; thread-per-row loops read half
+// of each with 32 lines a load.
 template <int NMAX>
 struct CholRefineSmem {
     double X[NMAX * kTriRhs];      // solution
