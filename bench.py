@@ -749,7 +749,7 @@ class TrsmVbatched:
 
     def dominant_kernel(self, q, stream, reps=20):
         ms = timed_restore(stream, lambda i: self.step(q, i), self.restore, reps) / reps
-        return {"kernel": "tri_panel_kernel<double,solve> (magmablas_dtrsm_vbatched_max_nocheck)", "ms": ms,
+        return {"kernel": "trsm_warp_kernel (magmablas_dtrsm_vbatched_max_nocheck)", "ms": ms,
                 "alg_bytes": self.bytes64, "tflops": self.flops / ms / 1e9}
 
     def e2e_setup(self):

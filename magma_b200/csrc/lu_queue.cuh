@@ -13,7 +13,9 @@
 // every team's shared memory fits its warps' shares; the chunk width only groups the
 // trailing columns, each element's updates keep their order. All paths apply the
 // unblocked dgetf2 operations in order, so factors, pivots, info and NoTrans solutions
-// are the same bits as the per-bucket kernels' and the oracle's. Counterparts in the
+// are the same bits as the oracle's and the per-bucket kernels', which update and solve on
+// the tensor cores (getrf_cluster.cu, getrs_tc.cu) and are the faster ones: the table's
+// default is one launch per bucket. Counterparts in the
 // reference: src/zgetrf_batched.cpp:222-351 (a launch sequence per call) and
 // magmablas/gemm_template_kernel_vbatched.cuh:53-54 (grids sized by the largest instance).
 #pragma once

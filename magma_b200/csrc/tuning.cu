@@ -1,9 +1,9 @@
 // tuning.cu -- kernel-variant table and its autotuner.
 //
 // The dispatchers of the variable-size GEMM (tile shape per size bucket), of
-// the mixed-precision solve (tensor-core or CUDA-core FP32 LU) and of the FP64
-// blocked LU (trailing update on the tensor cores or the FP64 pipe, per size
-// bucket) read one process-wide table. Defaults are built in; MAGMA_B200_TUNING=<file> loads a
+// the mixed-precision solve (tensor-core or CUDA-core FP32 LU) and of the
+// variable-size Cholesky and LU (one persistent launch or one per size bucket)
+// read one process-wide table. Defaults are built in; MAGMA_B200_TUNING=<file> loads a
 // saved table at first use; magma_b200_autotune() measures every variant on the
 // queue's device with synthetic problems of each bucket and keeps the fastest.
 // Every variant of a family computes bit-identical results (same fma order per
@@ -28,9 +28,9 @@ static std::once_flag g_once;
 
 // Built-in defaults: what magma_b200_autotune picked on B200s, with the GEMM tiles
 // checked on the C2 workload (20,000 instances, M, N, K in 8..128): FP64 16x16 / 32x32
-// CUDA-core tiles up to max(M, N) = 32 and the DMMA tile above (7.38 TF/s, against 6.94
+// CUDA-core tiles up to max(M, N) = 32 and the DMMA tile above (10.4 TF/s, against 6.94
 // with CUDA-core tiles throughout); FP32 CUDA-core tiles up to 64 and the tcgen05 tile
-// above (14.6 TF/s, against 10.7).
+// above (16.5 TF/s, against 10.7).
 static void set_defaults(TuningTable& t) {
     const int gemm[2][kGemmBuckets] = {{2, 1, 3, 3}, {2, 1, 1, 3}};
     for (int p = 0; p < 2; ++p)
